@@ -65,7 +65,7 @@ def default_candidates(ndim):
     else:
         tiles = [(64,), (256,), (1024,)]
     # visits per spread work item (a crowded tile is split over interleaved items)
-    return tiles, ([2048, 4096, 8192] if ndim == 3 else [1024, 2048, 4096])
+    return tiles, ([512, 2048, 4096, 8192] if ndim == 3 else [128, 512, 1024, 2048, 4096])
 
 
 def _time_pair(fwd, adj, iters):

@@ -1617,9 +1617,14 @@ __global__ void __launch_bounds__(Reg2Cfg<CPW>::NW * 32, Reg2Cfg<CPW>::MinBlocks
     }
 }
 
-// zero the tiles that several CTAs combine with atomics (planar grid)
+// Zero the tiles that several CTAs combine with atomics (planar grid): a CTA takes one
+// tile of kZeroCh channels, a thread one tile point (its position is formed once) and
+// walks the channels.  One CTA per tile for all channels left most of the chip idle on
+// plans with few crowded tiles and many channels (2D, 66 k samples x 256 channels:
+// 84 us; 64 channels x 8 frames: 23 us).
+constexpr int kZeroCh = 8;
 template <int D>
-__global__ void zero_tiles_kernel(Geom g, const OwnerItem *zero, int nch, float2 *grid, int basis) {
+__global__ void __launch_bounds__(256) zero_tiles_kernel(Geom g, const OwnerItem *zero, int nch, float2 *grid, int basis) {
     const OwnerItem it = zero[blockIdx.x];
     int org[3], text[3];
     for (int a = 0; a < 3; ++a) {
@@ -1635,13 +1640,14 @@ __global__ void zero_tiles_kernel(Geom g, const OwnerItem *zero, int nch, float2
     }
     const int grp = basis ? 0 : (it.frame < 0 ? 0 : it.frame);
     const int tp = text[0] * text[1] * text[2];
-    for (int e = threadIdx.x; e < tp * nch; e += blockDim.x) {
-        int ch = e / tp, pt = e - ch * tp;
+    const int c0 = blockIdx.y * kZeroCh, c1 = min(nch, c0 + kZeroCh);
+    for (int pt = threadIdx.x; pt < tp; pt += blockDim.x) {
         int t0 = pt % text[0], rest = pt / text[0], t1 = rest % text[1], t2 = rest / text[1];
         int64_t pos = pmod(org[0] + t0 - g.sh[0], g.nos[0]);
         if (D > 1) pos += (int64_t)pmod(org[1] + t1 - g.sh[1], g.nos[1]) * g.nos[0];
         if (D > 2) pos += (int64_t)pmod(org[2] + t2 - g.sh[2], g.nos[2]) * g.nos[0] * g.nos[1];
-        grid[((int64_t)grp * nch + ch) * g.gvol + pos] = make_float2(0.f, 0.f);
+        float2 *dst = grid + ((int64_t)grp * nch + c0) * g.gvol + pos;
+        for (int ch = c0; ch < c1; ++ch, dst += g.gvol) *dst = make_float2(0.f, 0.f);
     }
 }
 
@@ -1996,10 +2002,11 @@ int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void
             const OwnerItem *zero = basis ? p->d_zero_all : p->d_zero_frame;
             const int nzero = basis ? p->n_zero_all : p->n_zero_frame;
             if (nzero > 0) {
+                const dim3 zg((unsigned)nzero, (unsigned)((c.nch + kZeroCh - 1) / kZeroCh));
                 switch (p->g.ndim) {
-                    case 1: zero_tiles_kernel<1><<<nzero, 256, 0, s>>>(p->g, zero, c.nch, gridp, basis); break;
-                    case 2: zero_tiles_kernel<2><<<nzero, 256, 0, s>>>(p->g, zero, c.nch, gridp, basis); break;
-                    default: zero_tiles_kernel<3><<<nzero, 256, 0, s>>>(p->g, zero, c.nch, gridp, basis); break;
+                    case 1: zero_tiles_kernel<1><<<zg, 256, 0, s>>>(p->g, zero, c.nch, gridp, basis); break;
+                    case 2: zero_tiles_kernel<2><<<zg, 256, 0, s>>>(p->g, zero, c.nch, gridp, basis); break;
+                    default: zero_tiles_kernel<3><<<zg, 256, 0, s>>>(p->g, zero, c.nch, gridp, basis); break;
                 }
                 PFB_CHECK_LAUNCH();
             }

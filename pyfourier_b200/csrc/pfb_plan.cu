@@ -170,6 +170,22 @@ int default_tile(int ndim, int nos) {
     return std::max(1, std::min(t, nos));
 }
 
+// Visits per owner item before a crowded tile is split (its items interleave the
+// visits and are combined with atomics).  The spread's time is about a x chunk, the
+// serial chain of the fullest item, plus b x visits / chunk, the tile set-ups and
+// flushes of the split items: the best chunk grows with the square root of the number
+// of visits, about that of the samples.  Measured (spread kernel, us, at 128 / 256 /
+// 512 / 1024 / 2048 / 4096 visits per item): 2D radial 51 k samples x 8 channels 42 /
+// 45 / 49 / 73 / 112 / 218; 2D spiral 1.6 M x 64 2145 / 1793 / 1627 / 1534 / 1553 /
+// 1638; 3D radial 144 k x 5 151 / 144 / 151 / 192 / 293 / 483, 488 k x 10 568 / 512 /
+// 476 / 463 / 463 / 585, 8 M x 32 18119 / 14129 / 11998 / 10754 / 10339 / 10164.  The
+// upper end stays at 4096: longer items sum more visits serially in float32 per grid
+// point (8 M samples: the adjoint 4.7e-6 from float64 at 4096 visits, 1.15e-5 at 8192).
+int default_visits(int ndim, int64_t mtot) {
+    const double c = (ndim == 3 ? 1.4 : 0.85) * std::sqrt((double)mtot);
+    return (int)std::min(4096.0, std::max(128.0, c));
+}
+
 template <typename T>
 int dev_alloc(T **p, size_t count) {
     return pool_alloc(reinterpret_cast<void **>(p), (count == 0 ? 1 : count) * sizeof(T));
@@ -433,11 +449,7 @@ int plan_create(const float *coord, int ndim, int nframes, const int64_t *frame_
     p->max_bin = maxbin;
     int chunk = ndim == 3 ? 256 : 512;
     PFB_TRY_ST(rebuild_items(p, chunk));
-    // visits per owner item before a crowded tile is split (its items interleave the
-    // visits).  Longer items are faster but sum more visits serially in float32 per
-    // grid point: 3D radial 200^3 / 32 coils, spread 11.9 / 11.64 / 11.55 ms and the
-    // adjoint 4.9e-6 / 4.7e-6 / 1.15e-5 from float64 at 2048 / 4096 / 8192 visits
-    PFB_TRY_ST(build_owner_items(p, 4096));
+    PFB_TRY_ST(build_owner_items(p, default_visits(ndim, mtot)));
     PFB_TRY_ST(build_plan_taps(p, stream));
     // twiddle tables of the fused transform now, so that no apply allocates
     // (applies may be captured into CUDA graphs)
