@@ -27,7 +27,7 @@
 //                vals -> planar grid, owner-computes: one CTA per output tile (and
 //                channel group) accumulates the contributions of the samples whose
 //                first tap lies in the tile or in its 2^d - 1 lower neighbours, in
-//                registers (3D, and 2D above 16 channels) or in shared memory, then
+//                registers (3D, and 2D above 8 channels) or in shared memory, then
 //                stores the tile (plain stores; tiles too crowded for one CTA are
 //                split and combined with float2 atomics after a zeroing pass)
 //   crop_pl      planar grid -> image, cropped, deapodised, sum_l conj(C_l) (B0)
@@ -1738,7 +1738,6 @@ int launch_spread_reg2_t(const SpreadIL &P, int nitems, int nchunks, cudaStream_
 
 template <int WM>
 int launch_spread_reg2_w(const SpreadIL &P, int nitems, int nch, cudaStream_t s) {
-    if (nch <= 8) return launch_spread_reg2_t<WM, 8>(P, nitems, 1, s);
     if (nch <= 16) return launch_spread_reg2_t<WM, 16>(P, nitems, 1, s);
     return launch_spread_reg2_t<WM, 32>(P, nitems, (nch + 31) / 32, s);
 }
@@ -2035,10 +2034,12 @@ int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void
                                 : (wmv == 4 ? launch_spread_reg3_w<4>(S, nitems, c.nch, s)
                                             : launch_spread_reg3_w<8>(S, nitems, c.nch, s));
             }
-            if (p->g.ndim == 2 && p->g.tile[0] <= kReg2Tile && p->g.tile[1] <= kReg2Tile && c.nch > 16) {
-                // 2D register tiles (16 x 16 points), 32 channels per lane group (with
-                // fewer channels a CTA would have too few warps for the crowded tiles of
-                // radial trajectories: the shared-atomic kernel, 16 warps, is faster)
+            if (p->g.ndim == 2 && p->g.tile[0] <= kReg2Tile && p->g.tile[1] <= kReg2Tile && c.nch > 8) {
+                // 2D register tiles (16 x 16 points), 16 or 32 channels per lane group.  Up
+                // to 8 channels a CTA would have 2 warps, too few for a crowded tile's chain:
+                // the shared-atomic kernel, 16 warps, is faster there (205 k radial samples:
+                // 8 channels 123 us against 160 us, 12 channels 167 against 134 us, 16
+                // channels 175 against 136 us and, with width 6, 311 against 162 us)
                 return wmv == 1 ? launch_spread_reg2_w<1>(S, nitems, c.nch, s)
                                 : (wmv == 4 ? launch_spread_reg2_w<4>(S, nitems, c.nch, s)
                                             : launch_spread_reg2_w<8>(S, nitems, c.nch, s));
