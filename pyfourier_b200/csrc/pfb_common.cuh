@@ -11,9 +11,11 @@
 #include <cufft.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/pfb200.h"
@@ -121,6 +123,19 @@ struct ApplyDesc {
     int norm;               // 0: none, 1: ortho
 };
 
+// Taps per axis that the sample kernels are compiled for: 1 (Cartesian / sparse FFT), 4,
+// 6 or 8.  Width 6 is the default of the density compensation and of the Toeplitz plan;
+// walked as 8 taps it cost the 3D interp 512 taps for 216.
+inline int wm_of(const Geom &g) {
+    int w = g.w[0];
+    for (int a = 1; a < g.ndim; ++a) w = g.w[a] > w ? g.w[a] : w;
+    return w == 1 ? 1 : (w <= 4 ? 4 : (w <= 6 ? 6 : 8));
+}
+// Per-sample plan record of the spread and interp: D * WM kernel weights, then the D
+// wrapped first taps (int bits), padded to a multiple of 4 words so that every record
+// starts on a 16-byte boundary.
+__host__ __device__ constexpr int tap_rec(int D, int WM) { return (D * WM + D + 3) / 4 * 4; }
+
 // One axis of the fused FFT: a mixed-radix Stockham factorisation of n and
 // the offsets of each stage's twiddles exp(-2 pi i j q / (ns * radix)),
 // j < ns, 1 <= q < radix, in a device table.
@@ -159,8 +174,8 @@ struct pfb_plan {
     float *d_cos[pfb::kMaxDim] = {nullptr, nullptr, nullptr};  // bin-sorted oversampled coords
     int *d_perm = nullptr;       // sorted position -> global sample index
     int *d_iperm = nullptr;      // global sample index -> sorted position
-    float *d_wtap = nullptr;     // per sorted sample a record: D x WM kernel weights (WM = 4 for W <= 4,
-                                 // else 8), the D first taps x0 mod n_os, padded to 16 bytes
+    float *d_wtap = nullptr;     // per sorted sample a record: D x WM kernel weights (WM =
+                                 // wm_of), the D first taps x0 mod n_os, padded to 16 bytes
     int *d_xtap = nullptr;       // d_wtap + D * WM (first taps inside the records, not a separate buffer)
     int *d_sframe = nullptr;     // sorted position -> frame
     int *d_bin_start = nullptr;  // (nbins_total * ncode * F + 1) offsets into the sorted order
@@ -392,6 +407,11 @@ int fast_traj_grad(pfb_plan *p, const ApplyDesc &d, const float2 *img, const flo
 int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void *dst, void *ws, size_t wsb,
                float factor, bool accumulate, cudaStream_t s);
 int build_owner_items(pfb_plan *p, int chunk);
+// gather.cu: interleaved grid -> results of the sorted samples [M][nch]; the trajectory
+// gradient (values vt [M][B], weight applied)
+int launch_interp_il(const pfb_plan *p, const Chan &c, const float2 *grid, float2 *res, cudaStream_t s);
+int launch_traj_il(const pfb_plan *p, const Chan &c, const float2 *grid, const float2 *vt, const float2 *basis,
+                   const float2 *tB, float *grad, bool accumulate, cudaStream_t s);
 // per-sample kernel weights and first taps of the sorted samples (plan time)
 int build_plan_taps(pfb_plan *p, cudaStream_t s);
 void free_owner_items(pfb_plan *p);

@@ -17,8 +17,8 @@
 // Kernels:
 //   pad_pl       image (B, C, *N) -> planar grid, deapodised, zero-padded, times C_l (B0)
 //   transpose    planar grid -> interleaved grid
-//   interp_il    interleaved grid -> res[j][channel] (one warp per sample, lanes =
-//                channels x tap groups; x rows of the kernel box at 32 channels)
+//   gather_rows  interleaved grid -> res[j][channel] (pfb_gather.cu; also the
+//                trajectory gradient d/dk of sum_b Re(conj(A x)_b v_b))
 //   out_il       res -> k-space (B, M): sum over segments / coefficients with
 //                B_l(t) basis[f, k], density weight
 //   vals_il      k-space (B, M) -> vals[j][channel] in bin-sorted order, with the
@@ -31,7 +31,6 @@
 //                stores the tile (plain stores; tiles too crowded for one CTA are
 //                split and combined with float2 atomics after a zeroing pass)
 //   crop_pl      planar grid -> image, cropped, deapodised, sum_l conj(C_l) (B0)
-//   traj_il      d/dk of sum_b Re(conj(A x)_b v_b) (analytic Kaiser-Bessel derivative)
 #include <cmath>
 
 #include <type_traits>
@@ -42,7 +41,6 @@ namespace pfb {
 
 namespace {
 
-constexpr int kTileWarps = 8;        // warps per CTA of the sample kernels
 constexpr int kOutRows = 32;         // samples per CTA in the transposing kernels
 constexpr int kSpreadWarps = 16;     // warps per CTA of the spread
 
@@ -409,371 +407,8 @@ __global__ void __launch_bounds__(256) out_il_kernel(const SampIL P) {
 }
 
 
-// ------------------------------------------------------------------------------------
-// interp: one warp per bin-sorted sample, lanes = (tap group, channel)
-// ------------------------------------------------------------------------------------
-struct InterpIL {
-    Geom g;
-    const float *cos0, *cos1, *cos2;
-    const int *sframe;
-    int64_t mtot;
-    const float2 *grid;   // interleaved
-    float2 *res;          // [M][nch]
-    Chan ch;
-    int cw;               // lanes per channel chunk (power of two <= 32)
-    // trajectory gradient
-    const float2 *vt;     // [M][B] values (weight applied)
-    const float2 *basis;
-    const float2 *tB;
-    const int *perm;
-    const int64_t *frame_off;
-    int readout;
-    float chain[kMaxDim];
-    float *grad;          // (M, ndim) in original sample order
-    int accumulate;
-    const float *wtap;    // plan taps: records of tap_rec(D, WM) words (weights, then first taps mod n_os)
-    const int *xtap;
-};
-
-// Per-sample tap weights and FFT-layout positions, computed by lanes (axis, i)
-// and left in shared memory for the warp: w[a][i], p[a][i] (and dw/dc).
-template <int D, int WM, bool DERIV>
-__device__ __forceinline__ void warp_taps(const InterpIL &P, int64_t j, float *sw, int *sp, float *sd, int lane) {
-    if (lane < D * WM) {
-        int a = lane / WM, i = lane - a * WM;
-        const float *cs = a == 0 ? P.cos0 : (a == 1 ? P.cos1 : P.cos2);
-        float c = cs[j];
-        int w = P.g.w[a];
-        long long x0 = start_index(c, w, P.g.cart[a]);
-        float wv = 0.f, dv = 0.f;
-        if (P.g.cart[a]) {
-            wv = i == 0 ? 1.f : 0.f;
-        } else if (i < w) {
-            float halfw = 0.5f * (float)w;
-            float u = ((float)(x0 + i) - c) / halfw;
-            if (DERIV) {
-                float d;
-                wv = kb_eval_deriv(u, P.g.beta[a], &d);
-                dv = -d / halfw;
-            } else {
-                wv = kb_eval(u, P.g.beta[a]);
-            }
-        }
-        int q = pmod(x0 + i - P.g.sh[a], P.g.nos[a]);
-        sw[a * WM + i] = wv;
-        sp[a * WM + i] = q;
-        if (DERIV) sd[a * WM + i] = dv;
-    }
-}
-
 template <int D>
 __host__ __device__ constexpr int ipow(int b) { return D == 1 ? b : (D == 2 ? b * b : b * b * b); }
-
-// Per-sample plan record of the spread and interp: D * WM kernel weights, then
-// the D wrapped first taps (int bits), padded to a multiple of 4 words so that
-// every record starts on a 16-byte boundary (runs of records can be moved with
-// bulk copies).
-__host__ __device__ constexpr int tap_rec(int D, int WM) { return (D * WM + D + 3) / 4 * 4; }
-
-// Per-sample tap list in the warp's shared memory: the tap's offset and weight
-// for every tap of the WM^D box; taps beyond the kernel widths get weight 0 and
-// offset 0 (an in-bounds address).  The offset is the element offset point * nch
-// when that fits in 32 bits (WIDE = false), else the point index.  Lanes build
-// 32 taps at a time.
-template <int D, int WM, bool WIDE, typename WT>
-__device__ __forceinline__ void build_tap_list(const InterpIL &P, const float *sw, const int *sp, int nch,
-                                               int *s_off, WT *s_wt, int lane) {
-    constexpr int NT = ipow<D>(WM);
-    const int nx = P.g.nos[0], nxy = P.g.nos[0] * P.g.nos[1];
-    for (int t = lane; t < NT; t += 32) {
-        const int ix = t % WM, iy = (t / WM) % WM, iz = t / (WM * WM);
-        const bool ok = ix < P.g.w[0] && (D < 2 || iy < P.g.w[1]) && (D < 3 || iz < P.g.w[2]);
-        float w = 0.f;
-        int off = 0;
-        if (ok) {
-            w = sw[ix] * (D > 1 ? sw[WM + iy] : 1.f) * (D > 2 ? sw[2 * WM + iz] : 1.f);
-            off = sp[ix] + (D > 1 ? sp[WM + iy] * nx : 0) + (D > 2 ? sp[2 * WM + iz] * nxy : 0);
-            if (!WIDE) off *= nch;
-        }
-        s_off[t] = off;
-        if constexpr (sizeof(WT) == sizeof(float2))
-            s_wt[t] = make_float2(w, w);  // the broadcast operand of a packed FFMA2
-        else
-            s_wt[t] = w;
-    }
-}
-
-// Per-sample x rows of a 4-wide kernel box in the warp's shared memory, one row per
-// (y, z) tap pair: the row's offset (the y and z parts of the tap offset, scaled like
-// build_tap_list's) and its weight w_y * w_z as a (w, w) pair.  Lanes < rows build
-// one row each.  With the four x taps' positions and weights in registers, the
-// gather reads 12 bytes of shared memory per row of four taps instead of 12 bytes
-// per tap.
-template <int D, bool WIDE>
-__device__ __forceinline__ void build_rows(const InterpIL &P, const float *sw, const int *sp, int nch,
-                                           int *s_roff, float2 *s_rw, int lane) {
-    constexpr int WM = 4, NR = D == 3 ? 16 : 4;
-    if (lane < NR) {
-        const int iy = lane & 3, iz = lane >> 2;
-        const bool ok = iy < P.g.w[1] && (D < 3 || iz < P.g.w[2]);
-        float w = 0.f;
-        int off = 0;
-        if (ok) {
-            w = sw[WM + iy] * (D > 2 ? sw[2 * WM + iz] : 1.f);
-            off = sp[WM + iy] * P.g.nos[0] + (D > 2 ? sp[2 * WM + iz] * (P.g.nos[0] * P.g.nos[1]) : 0);
-            if (!WIDE) off *= nch;
-        }
-        s_roff[lane] = off;
-        s_rw[lane] = make_float2(w, w);
-    }
-}
-
-// XROWS: the launch has one channel per lane (channel chunks of 32) and a box 4
-// taps wide in 2D or 3D; the kernel then takes the x-row form and keeps no
-// per-tap list.  CH: the grid's channel count when fixed at compile time (x-row
-// form only), else 0.
-template <int D, int WM, bool WIDE, bool XROWS, int CH = 0>
-__global__ void __launch_bounds__(kTileWarps * 32, 3) interp_il_kernel(const InterpIL P) {
-    constexpr int NT = ipow<D>(WM);
-    // up to 64 taps the weights are kept as (w, w) pairs for FFMA2 and, with one
-    // channel per lane, the gather loop takes 4 taps per 16-byte offset load
-    constexpr bool PAIRS = NT <= 64;
-    constexpr bool VEC = PAIRS && NT % 4 == 0;
-    constexpr bool VEC16 = PAIRS && NT % 16 == 0;
-    constexpr bool ROWS = XROWS && PAIRS && WM == 4 && D >= 2;
-    static_assert(ROWS || !XROWS, "the x-row form needs a 2D / 3D box 4 taps wide");
-    static_assert(CH == 0 || (ROWS && !WIDE), "a compile-time channel count is for the 32-bit x-row form");
-    constexpr int NR = ROWS ? NT / 4 : 4;    // x rows of the box
-    constexpr int NL = ROWS ? 4 : NT;        // entries of the per-tap list
-    using WT = typename std::conditional<PAIRS, float2, float>::type;
-    __shared__ __align__(16) float s_w[kTileWarps][3 * WM];
-    __shared__ __align__(16) int s_p[kTileWarps][3 * WM];
-    __shared__ __align__(16) int s_off[kTileWarps][NL];
-    __shared__ __align__(16) WT s_wt[kTileWarps][NL];
-    __shared__ __align__(16) int s_roff[kTileWarps][NR];
-    __shared__ __align__(16) float2 s_rw[kTileWarps][NR];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cw = P.cw, lcw = log2i(cw), tg_n = 32 >> lcw;
-    const int cl = lane & (cw - 1), tg = lane >> lcw;
-    const int nch = P.ch.nch;
-    // each CTA takes a contiguous run of bin-sorted samples: its warps gather
-    // from the same few tiles, which stay in L1
-    const int64_t per = (P.mtot + gridDim.x - 1) / gridDim.x;
-    const int64_t jbeg = (int64_t)blockIdx.x * per, jend = min(P.mtot, jbeg + per);
-    // the plan taps (weights, first taps) and frame of the warp's next sample are
-    // loaded into registers while the current sample gathers
-    constexpr int DW = D * WM;
-    float pw = 0.f;
-    int px = 0, pf = 0;
-    auto fetch = [&](int64_t jj) {
-        if (jj < jend) {
-            if (lane < DW) {
-                pw = P.wtap[jj * tap_rec(D, WM) + lane];
-                px = P.xtap[jj * tap_rec(D, WM) + lane / WM];
-            }
-            pf = P.ch.K ? 0 : P.sframe[jj];
-        }
-    };
-    fetch(jbeg + warp);
-    for (int64_t j = jbeg + warp; j < jend; j += kTileWarps) {
-        if (lane < DW) {  // weights as stored, positions from the first tap x0 mod n_os
-            const int a = lane / WM, i = lane - a * WM;
-            s_w[warp][lane] = pw;
-            s_p[warp][lane] = pmod((long long)px + i - P.g.sh[a], P.g.nos[a]);
-        }
-        const int grp = pf;
-        fetch(j + kTileWarps);
-        __syncwarp();
-        const float2 *G = P.grid + (int64_t)grp * P.g.gvol * nch;
-        if constexpr (ROWS)
-            build_rows<D, WIDE>(P, s_w[warp], s_p[warp], nch, s_roff[warp], s_rw[warp], lane);
-        else
-            build_tap_list<D, WM, WIDE>(P, s_w[warp], s_p[warp], nch, s_off[warp], s_wt[warp], lane);
-        __syncwarp();
-        for (int c0 = 0; c0 < nch; c0 += cw) {
-            const int c = c0 + cl;
-            const float2 *Gc = G + (c < nch ? c : nch - 1);  // in-bounds address; result discarded
-            float2 acc = make_float2(0.f, 0.f);
-            if constexpr (ROWS) {
-                // 4 rows (16 gathers) in flight; each x position accumulates its
-                // column over the rows (weights w_y * w_z), the four columns are
-                // combined with the x weights at the end
-                const int4 px4 = *reinterpret_cast<const int4 *>(s_p[warp]);
-                float2 ax[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f),
-                                make_float2(0.f, 0.f)};
-                const int4 *ro4 = reinterpret_cast<const int4 *>(s_roff[warp]);
-                auto run = [&](auto addr) {
-#pragma unroll
-                    for (int rb = 0; rb < NR / 4; ++rb) {
-                        const int4 o = ro4[rb];
-                        const int oo[4] = {o.x, o.y, o.z, o.w};
-                        float2 v[16];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) v[4 * q + u] = __ldg(addr(oo[q], u));
-                        }
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const float2 wr = s_rw[warp][4 * rb + q];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) ax[u] = __ffma2_rn(wr, v[4 * q + u], ax[u]);
-                        }
-                    }
-                };
-                // with a compile-time channel count and the four x taps side by side
-                // (not split by the fftshift seam), a row is one pointer and its taps
-                // sit at fixed offsets from it
-                if (CH > 0 && px4.y == px4.x + 1 && px4.z == px4.x + 2 && px4.w == px4.x + 3) {
-                    const float2 *Gx0 = Gc + px4.x * CH;
-                    run([&](int o, int u) { return Gx0 + o + u * CH; });
-                } else {
-                    const float2 *Gx[4] = {WIDE ? Gc + (int64_t)px4.x * nch : Gc + px4.x * nch,
-                                           WIDE ? Gc + (int64_t)px4.y * nch : Gc + px4.y * nch,
-                                           WIDE ? Gc + (int64_t)px4.z * nch : Gc + px4.z * nch,
-                                           WIDE ? Gc + (int64_t)px4.w * nch : Gc + px4.w * nch};
-                    run([&](int o, int u) { return WIDE ? Gx[u] + (int64_t)o * nch : Gx[u] + o; });
-                }
-                const float4 wx4 = *reinterpret_cast<const float4 *>(s_w[warp]);
-                const int w0 = P.g.w[0];
-                const float wx1 = w0 > 1 ? wx4.y : 0.f, wx2 = w0 > 2 ? wx4.z : 0.f, wx3 = w0 > 3 ? wx4.w : 0.f;
-                acc = __fmul2_rn(make_float2(wx4.x, wx4.x), ax[0]);
-                acc = __ffma2_rn(make_float2(wx1, wx1), ax[1], acc);
-                acc = __ffma2_rn(make_float2(wx2, wx2), ax[2], acc);
-                acc = __ffma2_rn(make_float2(wx3, wx3), ax[3], acc);
-            } else {
-            if (VEC16 && tg_n == 1) {
-                // 16 gathers issued before their sums (more loads in flight per warp);
-                // taps summed in order 0, 1, 2, ...: the same sums as the loops below
-                const int4 *o4 = reinterpret_cast<const int4 *>(s_off[warp]);
-                const float4 *w4 = reinterpret_cast<const float4 *>(s_wt[warp]);
-                for (int t16 = 0; t16 < NT / 16; ++t16) {
-                    float2 v[16];
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const int4 o = o4[4 * t16 + g];
-                        const int oo[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            v[4 * g + u] = WIDE ? __ldg(Gc + (int64_t)oo[u] * nch) : __ldg(Gc + oo[u]);
-                    }
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const float4 wa = w4[2 * (4 * t16 + g)], wb = w4[2 * (4 * t16 + g) + 1];
-                        acc = __ffma2_rn(make_float2(wa.x, wa.y), v[4 * g + 0], acc);
-                        acc = __ffma2_rn(make_float2(wa.z, wa.w), v[4 * g + 1], acc);
-                        acc = __ffma2_rn(make_float2(wb.x, wb.y), v[4 * g + 2], acc);
-                        acc = __ffma2_rn(make_float2(wb.z, wb.w), v[4 * g + 3], acc);
-                    }
-                }
-            } else if (VEC && tg_n == 1) {
-                // taps in order 0, 1, 2, ...: the same sums as the loop below
-                const int4 *o4 = reinterpret_cast<const int4 *>(s_off[warp]);
-                const float4 *w4 = reinterpret_cast<const float4 *>(s_wt[warp]);
-#pragma unroll 4
-                for (int t4 = 0; t4 < NT / 4; ++t4) {
-                    const int4 o = o4[t4];
-                    const float4 wa = w4[2 * t4], wb = w4[2 * t4 + 1];
-                    float2 v[4];
-                    const int oo[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        v[u] = WIDE ? __ldg(Gc + (int64_t)oo[u] * nch) : __ldg(Gc + oo[u]);
-                    acc = __ffma2_rn(make_float2(wa.x, wa.y), v[0], acc);
-                    acc = __ffma2_rn(make_float2(wa.z, wa.w), v[1], acc);
-                    acc = __ffma2_rn(make_float2(wb.x, wb.y), v[2], acc);
-                    acc = __ffma2_rn(make_float2(wb.z, wb.w), v[3], acc);
-                }
-            } else {
-#pragma unroll 8
-                for (int t = tg; t < NT; t += tg_n) {
-                    const float2 v = WIDE ? __ldg(Gc + (int64_t)s_off[warp][t] * nch) : __ldg(Gc + s_off[warp][t]);
-                    if constexpr (PAIRS)
-                        acc = __ffma2_rn(s_wt[warp][t], v, acc);
-                    else
-                        acc = cfma(s_wt[warp][t], v, acc);
-                }
-            }
-            }
-            // reduce over tap groups (lanes that share the channel)
-            for (int off = cw; off < 32; off <<= 1) {
-                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, off);
-                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, off);
-            }
-            if (tg == 0 && c < nch) P.res[j * nch + c] = acc;
-        }
-        __syncwarp();
-    }
-}
-
-template <int D, int WM>
-__global__ void __launch_bounds__(kTileWarps * 32) traj_il_kernel(const InterpIL P) {
-    __shared__ float s_w[kTileWarps][3 * WM];
-    __shared__ float s_d[kTileWarps][3 * WM];
-    __shared__ int s_p[kTileWarps][3 * WM];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cw = P.cw, lcw = log2i(cw), tg_n = 32 >> lcw;
-    const int cl = lane & (cw - 1), tg = lane >> lcw;
-    const int nch = P.ch.nch, B = P.ch.B, Kc = P.ch.K ? P.ch.K : 1;
-    const int64_t nx = P.g.nos[0], nxy = (int64_t)P.g.nos[0] * P.g.nos[1];
-    const int wa[3] = {P.g.w[0], D > 1 ? P.g.w[1] : 1, D > 2 ? P.g.w[2] : 1};
-    const int64_t per = (P.mtot + gridDim.x - 1) / gridDim.x;
-    const int64_t jbeg = (int64_t)blockIdx.x * per, jend = min(P.mtot, jbeg + per);
-    for (int64_t j = jbeg + warp; j < jend; j += kTileWarps) {
-        warp_taps<D, WM, true>(P, j, s_w[warp], s_p[warp], s_d[warp], lane);
-        __syncwarp();
-        const int f = P.sframe[j];
-        const int gs = P.perm[j];
-        const int grp = P.ch.K ? 0 : f;
-        const int t = P.tB ? (int)((gs - P.frame_off[f]) % P.readout) : 0;
-        const float2 *G = P.grid + (int64_t)grp * P.g.gvol * nch;
-        float gacc[3] = {0.f, 0.f, 0.f};
-        for (int c0 = 0; c0 < nch; c0 += cw) {
-            const int c = c0 + cl;
-            float2 dsum[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            if (c < nch) {
-                for (int iz = 0; iz < wa[2]; ++iz) {
-                    const float wz = D > 2 ? s_w[warp][2 * WM + iz] : 1.f;
-                    const float dz = D > 2 ? s_d[warp][2 * WM + iz] : 0.f;
-                    const int64_t pz = D > 2 ? s_p[warp][2 * WM + iz] * nxy : 0;
-                    for (int iy = 0; iy < wa[1]; ++iy) {
-                        const float wy = D > 1 ? s_w[warp][WM + iy] : 1.f;
-                        const float dy = D > 1 ? s_d[warp][WM + iy] : 0.f;
-                        const int64_t rowp = pz + (D > 1 ? s_p[warp][WM + iy] * nx : 0);
-                        for (int ix = tg; ix < wa[0]; ix += tg_n) {
-                            const float wx = s_w[warp][ix], dx = s_d[warp][ix];
-                            const float2 h = __ldg(G + (rowp + s_p[warp][ix]) * nch + c);
-                            dsum[0] = cfma(wz * wy * dx, h, dsum[0]);
-                            if (D > 1) dsum[1] = cfma(wz * dy * wx, h, dsum[1]);
-                            if (D > 2) dsum[2] = cfma(dz * wy * wx, h, dsum[2]);
-                        }
-                    }
-                }
-                // channel factor B_l(t) basis[f, k] and the value v_b
-                const int k = c % Kc, lb = c / Kc, b = lb % B, l = lb / B;
-                float2 fac = make_float2(1.f, 0.f);
-                if (P.tB) fac = P.tB[(int64_t)l * P.readout + t];
-                if (P.ch.K) fac = cmul(fac, P.basis[(int64_t)f * P.ch.K + k]);
-                const float2 v = P.vt[j * B + b];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    float2 dd = cmul(dsum[a], fac);
-                    gacc[a] += dd.x * v.x + dd.y * v.y;  // Re(conj(D) v)
-                }
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-            for (int off = 16; off > 0; off >>= 1) gacc[a] += __shfl_xor_sync(0xffffffffu, gacc[a], off);
-        if (lane < D) {
-            float r = (lane == 0 ? gacc[0] : (lane == 1 ? gacc[1] : gacc[2])) * P.chain[lane];
-            float *dst = P.grad + (int64_t)gs * D + lane;
-            *dst = P.accumulate ? *dst + r : r;
-        }
-        __syncwarp();
-    }
-}
-
 
 // ------------------------------------------------------------------------------------
 // spread: owner-computes tiles
@@ -1663,12 +1298,6 @@ struct WsLayout {
     size_t gridp, gridi, samp, taps, work, total;
 };
 
-// taps per axis the kernels are compiled for: 1 (Cartesian / sparse FFT), 4 or 8
-int wm_of(const Geom &g) {
-    const int w = std::max(g.w[0], std::max(g.w[1], g.w[2]));
-    return w == 1 ? 1 : (w <= 4 ? 4 : 8);
-}
-
 int layout_ws(pfb_plan *p, const Chan &c, WsLayout *L, cufftHandle *h, size_t *wb) {
     const int64_t P = (int64_t)c.ngrp * c.nch;
     if (fft_fused_ready(p)) {
@@ -1685,32 +1314,6 @@ int layout_ws(pfb_plan *p, const Chan &c, WsLayout *L, cufftHandle *h, size_t *w
     L->taps = 0;  // the per-sample taps live in the plan
     L->work = up256(*wb);
     L->total = L->gridp + L->gridi + L->samp + L->taps + L->work;
-    return PFB_OK;
-}
-
-template <int D, int WM>
-int launch_interp_il_t(const InterpIL &P, int blocks, cudaStream_t s) {
-    // element offsets point * nch in 32 bits when the grid allows it
-    const bool wide = P.g.gvol * (int64_t)P.ch.nch >= (1LL << 31);
-    if constexpr (WM == 4 && D >= 2) {
-        if (P.cw == 32) {  // one channel per lane: the x-row form
-            if (!wide && P.ch.nch == 32) interp_il_kernel<D, WM, false, true, 32><<<blocks, kTileWarps * 32, 0, s>>>(P);
-            else if (!wide) interp_il_kernel<D, WM, false, true><<<blocks, kTileWarps * 32, 0, s>>>(P);
-            else interp_il_kernel<D, WM, true, true><<<blocks, kTileWarps * 32, 0, s>>>(P);
-            PFB_CHECK_LAUNCH();
-            return PFB_OK;
-        }
-    }
-    if (!wide) interp_il_kernel<D, WM, false, false><<<blocks, kTileWarps * 32, 0, s>>>(P);
-    else interp_il_kernel<D, WM, true, false><<<blocks, kTileWarps * 32, 0, s>>>(P);
-    PFB_CHECK_LAUNCH();
-    return PFB_OK;
-}
-
-template <int D, int WM>
-int launch_traj_il_t(const InterpIL &P, int blocks, cudaStream_t s) {
-    traj_il_kernel<D, WM><<<blocks, kTileWarps * 32, 0, s>>>(P);
-    PFB_CHECK_LAUNCH();
     return PFB_OK;
 }
 
@@ -1760,33 +1363,20 @@ int launch_spread_il_t(const SpreadIL &P, int nitems, int nchunks, size_t smem, 
     return PFB_OK;
 }
 
-int sample_blocks(int64_t mtot) {
-    int64_t b = (mtot + kTileWarps - 1) / kTileWarps;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148LL * 64));
+template <int D>
+int launch_spread_il(const SpreadIL &P, int wm, int nitems, int nchunks, size_t smem, cudaStream_t s) {
+    switch (wm) {
+        case 1: return launch_spread_il_t<D, 1>(P, nitems, nchunks, smem, s);
+        case 4: return launch_spread_il_t<D, 4>(P, nitems, nchunks, smem, s);
+        case 6: return launch_spread_il_t<D, 6>(P, nitems, nchunks, smem, s);
+        default: return launch_spread_il_t<D, 8>(P, nitems, nchunks, smem, s);
+    }
 }
 
 int flat_blocks(int64_t n) {
     int64_t b = (n + 255) / 256;
     return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148LL * 32));
 }
-
-void fill_interp(const pfb_plan *p, const Chan &c, InterpIL &P) {
-    P.g = p->g;
-    P.cos0 = p->d_cos[0];
-    P.cos1 = p->d_cos[1];
-    P.cos2 = p->d_cos[2];
-    P.sframe = p->d_sframe;
-    P.perm = p->d_perm;
-    P.mtot = p->mtot;
-    P.ch = c;
-    P.cw = std::min(32, pow2ceil(c.nch));
-    P.frame_off = p->d_frame_off;
-    P.readout = p->readout;
-    P.wtap = p->d_wtap;
-    P.xtap = p->d_xtap;
-    for (int a = 0; a < kMaxDim; ++a) P.chain[a] = (float)p->g.nos[a] / (float)p->g.n[a];
-}
-
 
 size_t tile_points(const pfb_plan *p) {
     return (size_t)p->g.tile[0] * (p->g.ndim > 1 ? p->g.tile[1] : 1) * (p->g.ndim > 2 ? p->g.tile[2] : 1);
@@ -1811,13 +1401,6 @@ int spread_cw(const pfb_plan *p, const Chan &c) {
     while (cw > 1 && spread_smem(p, cw) > kSpreadSmem) cw >>= 1;
     return cw;
 }
-
-#define PFB_DISPATCH_DW(ND, WMV, CALL1, CALL4, CALL8)                              \
-    switch (ND) {                                                                  \
-        case 1: return (WMV) == 1 ? CALL1(1) : ((WMV) == 4 ? CALL4(1) : CALL8(1)); \
-        case 2: return (WMV) == 1 ? CALL1(2) : ((WMV) == 4 ? CALL4(2) : CALL8(2)); \
-        default: return (WMV) == 1 ? CALL1(3) : ((WMV) == 4 ? CALL4(3) : CALL8(3)); \
-    }
 
 }  // namespace
 
@@ -1949,18 +1532,7 @@ int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void
         }
         case PFB_STAGE_INTERP: {
             if (p->mtot == 0) return PFB_OK;
-            InterpIL Q{};
-            fill_interp(p, c, Q);
-            Q.grid = gridi;
-            Q.res = samp;
-            int blocks = sample_blocks(p->mtot);
-#define PFB_I1(DD) launch_interp_il_t<DD, 1>(Q, blocks, s)
-#define PFB_I4(DD) launch_interp_il_t<DD, 4>(Q, blocks, s)
-#define PFB_I8(DD) launch_interp_il_t<DD, 8>(Q, blocks, s)
-            PFB_DISPATCH_DW(p->g.ndim, wmv, PFB_I1, PFB_I4, PFB_I8)
-#undef PFB_I1
-#undef PFB_I4
-#undef PFB_I8
+            return launch_interp_il(p, c, gridi, samp, s);
         }
         case PFB_STAGE_OUT:
         case PFB_STAGE_VALS: {
@@ -2030,9 +1602,12 @@ int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void
                 p->g.tile[2] <= kRegTile) {
                 // register-tile form: channels in groups of 8, 16 or 32 per block, no
                 // shared atomics
-                return wmv == 1 ? launch_spread_reg3_w<1>(S, nitems, c.nch, s)
-                                : (wmv == 4 ? launch_spread_reg3_w<4>(S, nitems, c.nch, s)
-                                            : launch_spread_reg3_w<8>(S, nitems, c.nch, s));
+                switch (wmv) {
+                    case 1: return launch_spread_reg3_w<1>(S, nitems, c.nch, s);
+                    case 4: return launch_spread_reg3_w<4>(S, nitems, c.nch, s);
+                    case 6: return launch_spread_reg3_w<6>(S, nitems, c.nch, s);
+                    default: return launch_spread_reg3_w<8>(S, nitems, c.nch, s);
+                }
             }
             if (p->g.ndim == 2 && p->g.tile[0] <= kReg2Tile && p->g.tile[1] <= kReg2Tile && c.nch > 8) {
                 // 2D register tiles (16 x 16 points), 16 or 32 channels per lane group.  Up
@@ -2040,19 +1615,20 @@ int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void
                 // the shared-atomic kernel, 16 warps, is faster there (205 k radial samples:
                 // 8 channels 123 us against 160 us, 12 channels 167 against 134 us, 16
                 // channels 175 against 136 us and, with width 6, 311 against 162 us)
-                return wmv == 1 ? launch_spread_reg2_w<1>(S, nitems, c.nch, s)
-                                : (wmv == 4 ? launch_spread_reg2_w<4>(S, nitems, c.nch, s)
-                                            : launch_spread_reg2_w<8>(S, nitems, c.nch, s));
+                switch (wmv) {
+                    case 1: return launch_spread_reg2_w<1>(S, nitems, c.nch, s);
+                    case 4: return launch_spread_reg2_w<4>(S, nitems, c.nch, s);
+                    case 6: return launch_spread_reg2_w<6>(S, nitems, c.nch, s);
+                    default: return launch_spread_reg2_w<8>(S, nitems, c.nch, s);
+                }
             }
             const size_t smem = spread_smem(p, S.cw);
             const int nchunks = (c.nch + S.cw - 1) / S.cw;
-#define PFB_S1(DD) launch_spread_il_t<DD, 1>(S, nitems, nchunks, smem, s)
-#define PFB_S4(DD) launch_spread_il_t<DD, 4>(S, nitems, nchunks, smem, s)
-#define PFB_S8(DD) launch_spread_il_t<DD, 8>(S, nitems, nchunks, smem, s)
-            PFB_DISPATCH_DW(p->g.ndim, wmv, PFB_S1, PFB_S4, PFB_S8)
-#undef PFB_S1
-#undef PFB_S4
-#undef PFB_S8
+            switch (p->g.ndim) {
+                case 1: return launch_spread_il<1>(S, wmv, nitems, nchunks, smem, s);
+                case 2: return launch_spread_il<2>(S, wmv, nitems, nchunks, smem, s);
+                default: return launch_spread_il<3>(S, wmv, nitems, nchunks, smem, s);
+            }
         }
         default:
             return fail(PFB_ERR_INVALID, "unknown stage");
@@ -2114,23 +1690,7 @@ int fast_traj_grad(pfb_plan *p, const ApplyDesc &d, const float2 *img, const flo
     PFB_RAISE_SMEM(vals_il_kernel, (int)smem);
     vals_il_kernel<<<(unsigned)((p->mtot + V.rows - 1) / V.rows), 256, smem, s>>>(V);
     PFB_CHECK_LAUNCH();
-    InterpIL Q{};
-    fill_interp(p, c, Q);
-    Q.grid = gridi;
-    Q.vt = samp;
-    Q.basis = d.basis;
-    Q.tB = d.b0_time;
-    Q.grad = grad;
-    Q.accumulate = accumulate ? 1 : 0;
-    const int wmv = wm_of(p->g);
-    int blocks = sample_blocks(p->mtot);
-#define PFB_T1(DD) launch_traj_il_t<DD, 1>(Q, blocks, s)
-#define PFB_T4(DD) launch_traj_il_t<DD, 4>(Q, blocks, s)
-#define PFB_T8(DD) launch_traj_il_t<DD, 8>(Q, blocks, s)
-    PFB_DISPATCH_DW(p->g.ndim, wmv, PFB_T1, PFB_T4, PFB_T8)
-#undef PFB_T1
-#undef PFB_T4
-#undef PFB_T8
+    return launch_traj_il(p, c, gridi, samp, d.basis, d.b0_time, grad, accumulate, s);
 }
 
 // ------------------------------------------------------------------------------------
@@ -2244,10 +1804,13 @@ int build_plan_taps(pfb_plan *p, cudaStream_t s) {
         case 21: taps_prep_kernel<2, 1><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         case 31: taps_prep_kernel<3, 1><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         case 14: taps_prep_kernel<1, 4><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
+        case 16: taps_prep_kernel<1, 6><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         case 18: taps_prep_kernel<1, 8><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         case 24: taps_prep_kernel<2, 4><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
+        case 26: taps_prep_kernel<2, 6><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         case 28: taps_prep_kernel<2, 8><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         case 34: taps_prep_kernel<3, 4><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
+        case 36: taps_prep_kernel<3, 6><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
         default: taps_prep_kernel<3, 8><<<tb, 256, 0, s>>>(p->g, p->d_cos[0], p->d_cos[1], p->d_cos[2], p->mtot, w, x); break;
     }
     PFB_CHECK_LAUNCH();
