@@ -10,8 +10,10 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpfb200.so")
 SOURCES = ["pfb_capi.cu", "pfb_plan.cu", "pfb_spread.cu", "pfb_interp.cu", "pfb_glue.cu", "pfb_noalloc.cu", "pfb_fast.cu",
-           "pfb_gather.cu",
-           "pfb_fft.cu", "pfb_dcf.cu", "pfb_grog.cu", "pfb_psf.cu", "pfb_sort.cu", "pfb_pool.cu"]
+           "pfb_gather.cu", "pfb_fft.cu", "pfb_fft_cols_in.cu", "pfb_fft_cols_fwd.cu", "pfb_fft_cols_inv.cu",
+           "pfb_fft_cols_out.cu", "pfb_fft_cols_big.cu", "pfb_fft_rows.cu", "pfb_fft_tma.cu",
+           "pfb_dcf.cu", "pfb_grog.cu", "pfb_psf.cu", "pfb_sort.cu", "pfb_pool.cu"]
+HEADERS = ["pfb_common.cuh", "pfb_fft.cuh", "pfb_fft_passes.cuh", "pfb_fft_cols.cuh"]
 
 
 def nvcc_path():
@@ -21,7 +23,7 @@ def nvcc_path():
 
 def build(force=False, verbose=False, extra_flags=()):
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
-    deps = srcs + [os.path.join(CSRC, "pfb_common.cuh"), os.path.join(ROOT, "include", "pfb200.h")]
+    deps = srcs + [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", "pfb200.h")]
     if not force and os.path.exists(LIB):
         t = os.path.getmtime(LIB)
         if all(os.path.getmtime(d) <= t for d in deps):

@@ -136,16 +136,18 @@ inline int wm_of(const Geom &g) {
 // starts on a 16-byte boundary.
 __host__ __device__ constexpr int tap_rec(int D, int WM) { return (D * WM + D + 3) / 4 * 4; }
 
-// One axis of the fused FFT: a mixed-radix Stockham factorisation of n and
-// the offsets of each stage's twiddles exp(-2 pi i j q / (ns * radix)),
-// j < ns, 1 <= q < radix, in a device table.
-constexpr int kFftMaxStages = 16;
+// One axis of the fused FFT: the stages of its n-point transform and the offsets of their
+// twiddles exp(-2 pi i j q / (ns * radix)), 1 <= q < radix, j < ns (by q), in a device
+// table; a stage whose radix is a prime above 13 also has its roots there.
+constexpr int kFftMaxStages = 8;
 struct FftAxis {
     int n = 0, nst = 0;
     int radix[kFftMaxStages] = {};
     int ns[kFftMaxStages] = {};
     int twoff[kFftMaxStages] = {};
-    unsigned magic[kFftMaxStages] = {};  // floor(i / ns) = umulhi(i, magic) for i < 2^16 (ns > 1)
+    int rootoff[kFftMaxStages] = {};
+    unsigned magic[kFftMaxStages] = {};    // floor(i / ns) = umulhi(i, magic) for i < 2^16 (ns > 1)
+    unsigned magic_m[kFftMaxStages] = {};  // the same for n / radix
     const float2 *tw = nullptr;
 };
 

@@ -1,0 +1,10 @@
+// Column passes: the middle of a forward transform.
+#include "pfb_fft_cols.cuh"
+
+namespace pfb {
+namespace fft {
+
+template int launch_col_mode<kForward, false>(const ColPass &, cudaStream_t);
+
+}  // namespace fft
+}  // namespace pfb

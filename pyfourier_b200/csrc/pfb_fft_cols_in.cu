@@ -1,0 +1,10 @@
+// Column passes: the image side of a forward transform.
+#include "pfb_fft_cols.cuh"
+
+namespace pfb {
+namespace fft {
+
+template int launch_col_mode<kImageIn, false>(const ColPass &, cudaStream_t);
+
+}  // namespace fft
+}  // namespace pfb
