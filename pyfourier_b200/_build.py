@@ -11,9 +11,9 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libpfb200.so")
 SOURCES = ["pfb_capi.cu", "pfb_plan.cu", "pfb_spread.cu", "pfb_interp.cu", "pfb_glue.cu", "pfb_noalloc.cu", "pfb_fast.cu",
            "pfb_gather.cu", "pfb_fft.cu", "pfb_fft_cols_in.cu", "pfb_fft_cols_fwd.cu", "pfb_fft_cols_inv.cu",
-           "pfb_fft_cols_out.cu", "pfb_fft_cols_big.cu", "pfb_fft_rows.cu", "pfb_fft_tma.cu",
-           "pfb_dcf.cu", "pfb_grog.cu", "pfb_psf.cu", "pfb_sort.cu", "pfb_pool.cu"]
-HEADERS = ["pfb_common.cuh", "pfb_fft.cuh", "pfb_fft_passes.cuh", "pfb_fft_cols.cuh"]
+           "pfb_fft_cols_out.cu", "pfb_fft_cols_big.cu", "pfb_fft_rows.cu", "pfb_fft_tma.cu", "pfb_fft_gram.cu",
+           "pfb_fft_gram_big.cu", "pfb_dcf.cu", "pfb_grog.cu", "pfb_psf.cu", "pfb_sort.cu", "pfb_pool.cu"]
+HEADERS = ["pfb_common.cuh", "pfb_fft.cuh", "pfb_fft_passes.cuh", "pfb_fft_cols.cuh", "pfb_fft_gram.cuh"]
 
 
 def nvcc_path():

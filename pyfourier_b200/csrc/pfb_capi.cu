@@ -155,6 +155,25 @@ struct pfb_gram {
     int lowrank = 0;
     int nseg = 1;          // B0 time segments (one kernel each)
     float2 *d_T = nullptr;
+    int fused = 0;         // every axis is taken by the fused passes (2D and 3D)
+    FftAxis ax[3];
+    float2 *d_tw = nullptr;
+    GramFused desc() const {
+        GramFused f{};
+        f.ndim = ndim;
+        f.K = K;
+        f.lowrank = lowrank;
+        f.nseg = nseg;
+        for (int a = 0; a < 3; ++a) {
+            f.n[a] = n[a];
+            f.nos[a] = nos[a];
+        }
+        f.nvol = nvol;
+        f.gvol = gvol;
+        f.ax = ax;
+        f.kern = d_T;
+        return f;
+    }
     std::mutex fft_mu;
     std::map<int64_t, cufftHandle> fft_plans;
     std::map<int64_t, size_t> fft_work;
@@ -513,6 +532,7 @@ int pfb_gram_create(int ndim, const int *shape, const int *os_shape, int ncoeff,
         delete g;
         return fail(PFB_ERR_CUDA, std::string("kernel copy: ") + cudaGetErrorString(e));
     }
+    if (ndim >= 2) g->fused = fft_axes(ndim, g->nos, g->ax, &g->d_tw);
     *out = g;
     return PFB_OK;
 }
@@ -524,7 +544,8 @@ int pfb_gram_destroy(pfb_gram *g) {
         std::lock_guard<std::mutex> lk(g->fft_mu);
         for (auto &kv : g->fft_plans) cufftDestroy(kv.second);
     }
-    cudaFree(g->d_T);
+    cudaFree(g->d_T);  // synchronises the device
+    pool_free(g->d_tw, 0);
     delete g;
     return PFB_OK;
 }
@@ -532,6 +553,10 @@ int pfb_gram_destroy(pfb_gram *g) {
 int pfb_gram_workspace_size(pfb_gram *g, int64_t batch, size_t *bytes) {
     if (!g || !bytes || batch < 1) return fail(PFB_ERR_INVALID, "bad argument");
     DeviceGuard dg(g->device);
+    if (g->fused) {
+        *bytes = gram_fused_workspace(g->desc(), batch);
+        return PFB_OK;
+    }
     int64_t P = (int64_t)g->nseg * batch * g->K;
     cufftHandle h;
     size_t wb = 0;
@@ -551,6 +576,12 @@ int pfb_gram_apply(pfb_gram *g, const void *image, void *out, int64_t batch, con
     if (batch == 0) return PFB_OK;
     DeviceGuard dg(g->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (g->fused) {
+        const GramFused f = g->desc();
+        if (workspace_bytes < gram_fused_workspace(f, batch)) return fail(PFB_ERR_WORKSPACE, "workspace too small");
+        return gram_fused_apply(f, static_cast<const float2 *>(image), static_cast<float2 *>(out), batch,
+                                static_cast<const float2 *>(b0_space), workspace, s);
+    }
     const int L = g->nseg;
     const int64_t bk = batch * g->K;  // image planes
     const int64_t P = L * bk;         // grid planes (segment-major)

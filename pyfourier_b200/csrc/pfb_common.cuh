@@ -431,7 +431,22 @@ void pool_free(void *p, cudaStream_t s);
 int counting_sort_pairs(const int *keys, const int *vals, int *keys_out, int *vals_out, int64_t n, int end_bit,
                         void *temp, size_t temp_bytes, cudaStream_t s);
 
-// fused pruned FFT (pfb_fft.cu): 1 when it applies to the plan (tables ready)
+// fused pruned FFT (pfb_fft.cu).  The Gram: 1 and the axes with a device twiddle table
+// (pool memory of the current device) when every axis is taken, else 0.
+int fft_axes(int ndim, const int *nos, FftAxis *ax, float2 **d_tw);
+// Gram apply: images [plane][*n] -> out through grids of N rows (see pfb_fft_gram.cu);
+// planes = segments x batch x K; ws: gram_fused_workspace bytes
+struct GramFused {
+    int ndim, K, lowrank, nseg;
+    int n[3], nos[3];
+    int64_t nvol, gvol;
+    const FftAxis *ax;
+    const float2 *kern;
+};
+size_t gram_fused_workspace(const GramFused &g, int64_t batch);
+int gram_fused_apply(const GramFused &g, const float2 *image, float2 *out, int64_t batch, const float2 *Cl, void *ws,
+                     cudaStream_t s);
+// 1 when it applies to the plan (tables ready)
 int fft_fused_ready(pfb_plan *p);
 void fft_fused_free(pfb_plan *p);
 // forward passes: 0 image -> first intermediate, 1 middle (3D only), 2 -> interleaved grid

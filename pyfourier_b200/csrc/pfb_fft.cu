@@ -44,6 +44,11 @@ int launch_col(const ColPass &P, int mode, cudaStream_t s) {
     }
 }
 
+int launch_gram_rows(const GramRows &P, cudaStream_t s) {
+    if (P.batch == 0 || P.rows == 0) return PFB_OK;
+    return big_plan(P.fa) ? launch_gram_rows_t<true>(P, s) : launch_gram_rows_t<false>(P, s);
+}
+
 }  // namespace fft
 namespace {
 
@@ -179,7 +184,7 @@ bool make_axis(int n, bool rows, FftAxis *fa, std::vector<float2> &tw, size_t *b
 
 }  // namespace
 
-static int fft_axes(int ndim, const int *nos, FftAxis *ax, float2 **d_tw) {
+int fft_axes(int ndim, const int *nos, FftAxis *ax, float2 **d_tw) {
     *d_tw = nullptr;
     int large = 0;  // axes with a prime factor above kMaxPrime
     for (int a = 0; a < ndim; ++a) {
@@ -401,6 +406,107 @@ int fft_fused_adj(pfb_plan *p, int pass, const Chan &c, int C, float2 *img, cons
         Q.src = gridi;
     }
     return launch_col(Q, kImageOut, s);
+}
+
+namespace {
+// the Gram's grids: [plane][n2][N1][N0] after the z pass (3D) and [plane][n2][n1][N0]
+// before the rows; a dense Gram (N = n on every axis, one segment) works in the output
+bool gram_dense(const GramFused &g) {
+    bool d = g.nseg == 1;
+    for (int a = 0; a < g.ndim; ++a) d = d && g.n[a] == g.nos[a];
+    return d;
+}
+size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+}  // namespace
+
+size_t gram_fused_workspace(const GramFused &g, int64_t batch) {
+    if (gram_dense(g)) return 256;
+    const int64_t P = (int64_t)g.nseg * batch * g.K, n2 = g.ndim == 3 ? g.nos[2] : 1;
+    const size_t rows = up256((size_t)(P * n2 * g.nos[1] * g.n[0]) * sizeof(float2));
+    return rows + (g.ndim == 3 ? up256((size_t)(P * n2 * g.n[1] * g.n[0]) * sizeof(float2)) : 0);
+}
+
+int gram_fused_apply(const GramFused &g, const float2 *image, float2 *out, int64_t batch, const float2 *Cl, void *ws,
+                     cudaStream_t s) {
+    const int64_t bk = batch * g.K, P = g.nseg * bk;
+    const int64_t N0 = g.n[0], N1 = g.n[1], n1 = g.nos[1], n2 = g.ndim == 3 ? g.nos[2] : 1;
+    if (P >= (1LL << 31) || n1 * n2 >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many planes for the Gram");
+    const bool dense = gram_dense(g);
+    float2 *rows = dense ? out : static_cast<float2 *>(ws);
+    float2 *zgrid = dense ? out : reinterpret_cast<float2 *>(static_cast<char *>(ws) +
+                                                             up256((size_t)(P * n2 * n1 * N0) * sizeof(float2)));
+    // images and segments as channels of one group; no fftshift rotation (the embedding
+    // sits at the origin)
+    ColPass Q{};
+    Q.X = (int)N0;
+    Q.ch.nch = (int)P;
+    Q.ch.ngrp = 1;
+    Q.ch.B = (int)bk;
+    Q.ch.L = g.nseg;
+    Q.C = 1;
+    Q.nvol = g.nvol;
+    Q.Cl = Cl;
+    Q.factor = 1.f;
+    // the outermost axis, on the image side
+    const int za = g.ndim - 1;
+    Q.fa = g.ax[za];
+    Q.lin = Q.lout = g.n[za];
+    Q.nmid = g.ndim == 3 ? (int)N1 : 1;
+    ColPass F = Q, I = Q;
+    const int64_t zmid = g.ndim == 3 ? N0 : 0, zax = g.ndim == 3 ? N1 * N0 : N0, zplane = g.nos[za] * zax;
+    F.nplanes = (int)P;
+    F.in_mid = F.out_mid = I.in_mid = I.out_mid = zmid;
+    F.in_ax = F.out_ax = I.in_ax = I.out_ax = zax;
+    F.out_plane = I.in_plane = zplane;
+    F.lout = g.nos[za];
+    I.lin = g.nos[za];
+    I.nplanes = (int)bk;
+    float2 *z = g.ndim == 3 ? zgrid : rows;
+    F.src = image;
+    F.dst = z;
+    I.src = z;
+    I.dst = out;
+    I.factor = (float)(1.0 / (double)g.gvol);  // of the two transforms
+    int st = launch_col(F, kImageIn, s);
+    if (st) return st;
+    ColPass Y{};
+    if (g.ndim == 3) {
+        Y.fa = g.ax[1];
+        Y.X = (int)N0;
+        Y.nplanes = (int)P;
+        Y.nmid = (int)n2;
+        Y.in_ax = Y.out_ax = N0;
+        Y.lin = (int)N1;
+        Y.lout = (int)n1;
+        Y.in_plane = n2 * N1 * N0;
+        Y.in_mid = N1 * N0;
+        Y.out_plane = n2 * n1 * N0;
+        Y.out_mid = n1 * N0;
+        Y.src = zgrid;
+        Y.dst = rows;
+        if ((st = launch_col(Y, kForward, s))) return st;
+    }
+    GramRows R{};
+    R.fa = g.ax[0];
+    R.N0 = (int)N0;
+    R.rows = (int)(n1 * n2);
+    R.K = g.K;
+    R.lowrank = g.lowrank;
+    R.batch = (int)batch;
+    R.nseg = g.nseg;
+    R.gvol = g.gvol;
+    R.kern = g.kern;
+    R.grid = rows;
+    if ((st = launch_gram_rows(R, s))) return st;
+    if (g.ndim == 3) {
+        std::swap(Y.lin, Y.lout);
+        std::swap(Y.in_plane, Y.out_plane);
+        std::swap(Y.in_mid, Y.out_mid);
+        Y.src = rows;
+        Y.dst = zgrid;
+        if ((st = launch_col(Y, kInverse, s))) return st;
+    }
+    return launch_col(I, kImageOut, s);
 }
 
 }  // namespace pfb

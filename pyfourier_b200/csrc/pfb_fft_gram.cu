@@ -1,0 +1,10 @@
+// The Gram's middle pass.
+#include "pfb_fft_gram.cuh"
+
+namespace pfb {
+namespace fft {
+
+template int launch_gram_rows_t<false>(const GramRows &, cudaStream_t);
+
+}  // namespace fft
+}  // namespace pfb

@@ -1,0 +1,10 @@
+// The Gram's middle pass of the stage plans with a radix above 16.
+#include "pfb_fft_gram.cuh"
+
+namespace pfb {
+namespace fft {
+
+template int launch_gram_rows_t<true>(const GramRows &, cudaStream_t);
+
+}  // namespace fft
+}  // namespace pfb

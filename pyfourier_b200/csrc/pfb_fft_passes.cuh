@@ -84,13 +84,28 @@ struct RowPass {
     Div dt, dchunk, dyb, dz, dcpt, dunit;  // dunit: store units of a full tile
 };
 
+// The Gram's middle pass (pfb_fft_gram.cu): rows of the grid, N0 of n points held, in place
+struct GramRows {
+    FftAxis fa;
+    int N0, rows;             // points held per row; rows of the grid (n1 x n2)
+    int K, lowrank, batch, nseg;
+    int64_t gvol;             // points of the kernel per segment (and plane)
+    const float2 *kern;       // K x K matrices per point, or K planes; a leading segment axis
+    float2 *grid;             // [segment][batch][K][row][N0]
+    int V, T, nbv, nbg;       // set by the launch: vectors and threads, batch items per CTA, groups
+    Div dt, dbg, dk, drow;
+};
+int launch_gram_rows(const GramRows &P, cudaStream_t s);
+
 // TMA forms (pfb_fft_tma.cu): 1 if launched, 0 to take the direct form, or an error
 int launch_col_tma(const ColPass &P, int pass, cudaStream_t s);
 int launch_row_tma(const RowPass &P, bool inv, cudaStream_t s);
 int launch_col(const ColPass &P, int mode, cudaStream_t s);
-// one instantiation per file (pfb_fft_cols_*.cu), so that they compile side by side
+// one instantiation per file (pfb_fft_cols_*.cu, pfb_fft_gram*.cu), so that they compile side by side
 template <int MODE, bool BIG>
 int launch_col_mode(const ColPass &P, cudaStream_t s);
+template <bool BIG>
+int launch_gram_rows_t(const GramRows &P, cudaStream_t s);
 int launch_row(const RowPass &P, bool inv, cudaStream_t s);
 
 // Threads per vector of a CTA with nv vectors: the count (64 to kMaxThreads threads) that
