@@ -759,6 +759,74 @@ struct RegCfg {
 
 
 
+// Issues the asynchronous copies of batch bb (nb visits of nbat batches) of a register
+// spread: values [nb][CPW], plan records [nb][REC] and neighbour deltas [nb].  A warp takes
+// rounds of 32 samples (warp, warp + NW, ... in units of 32): lane l resolves sample
+// q0 + l (its sorted position and neighbour delta), then the warp copies the round's plan
+// records and value rows in 16-byte pieces, consecutive lanes on consecutive pieces of a
+// row.  (2D with one warp per sample and three per-lane copy streams: 74 instructions per
+// visit; 1.6 M samples x 64 channels 1529 -> 1351 us, 176^2 x 15 coils 25 -> 22 us; 6-wide and 96
+// channels over 64 frames unchanged within 1 %.)
+template <int CPW, int REC, int NR, int NW>
+__device__ __forceinline__ void stage_samples(const SpreadIL &P, const OwnerItem &it, int vs, int bb, int nbat, int nb,
+                                              const int *s_pre, const int *s_beg, const int *s_dlt, int c0, int warp,
+                                              int lane, float2 *rv, int *rr, int *rd) {
+    const int nch = P.ch.nch;
+    for (int q0 = warp * 32; q0 < nb; q0 += NW * 32) {
+        const int q = q0 + lane, nq = min(32, nb - q0);
+        int j = 0;
+        if (q < nb) {
+            // batch bb takes visits bb, bb + nbat, bb + 2 nbat, ...: every batch
+            // mixes the neighbour ranges, so all warps find work in it
+            const int v = it.v0 + (bb + q * nbat) * vs;
+            // range: the last one whose prefix is <= v (empty ranges share the
+            // prefix of the next one and are skipped)
+            int lo = 0, hi = NR;
+            while (hi - lo > 1) {
+                const int m = (lo + hi) >> 1;
+                if (s_pre[m] <= v) lo = m;
+                else hi = m;
+            }
+            j = s_beg[lo] + (v - s_pre[lo]);
+            rd[q] = s_dlt[lo];
+        }
+        // plan records: REC / 4 pieces per sample.  Lanes past the round's last
+        // piece copy nothing (a zero-size copy still writes its destination)
+        constexpr int RP = REC / 4;
+        for (int e0 = 0; e0 < nq * RP; e0 += 32) {
+            const int e = e0 + lane;
+            const bool in = e < nq * RP;
+            const int sq = in ? e / RP : 0, part = e - sq * RP;
+            const int js = __shfl_sync(0xffffffffu, j, sq);
+            if (in) cp_async16(rr + (q0 + sq) * REC + 4 * part, P.wtap + (int64_t)js * REC + 4 * part, true);
+        }
+        // value rows: channels c0 .. c0 + CPW - 1, zero-filled past nch; lanes past
+        // the round's last piece copy nothing
+        if (nch % 2 == 0) {
+            constexpr int VP = CPW / 2;  // 16-byte pieces (two channels) per row
+            for (int e0 = 0; e0 < nq * VP; e0 += 32) {
+                const int e = e0 + lane;
+                const bool in = e < nq * VP;
+                const int sq = in ? e / VP : 0, part = e - sq * VP;
+                const int js = __shfl_sync(0xffffffffu, j, sq);
+                const int ch = c0 + 2 * part;
+                const bool ok = ch < nch;
+                if (in) cp_async16(rv + (q0 + sq) * CPW + 2 * part, P.vals + (ok ? (int64_t)js * nch + ch : 0), ok);
+            }
+        } else {
+            for (int e0 = 0; e0 < nq * CPW; e0 += 32) {
+                const int e = e0 + lane;
+                const bool in = e < nq * CPW;
+                const int sq = in ? e / CPW : 0, part = e - sq * CPW;
+                const int js = __shfl_sync(0xffffffffu, j, sq);
+                const int ch = c0 + part;
+                const bool ok = ch < nch;
+                if (in) cp_async8(rv + (q0 + sq) * CPW + part, P.vals + (ok ? (int64_t)js * nch + ch : 0), ok);
+            }
+        }
+    }
+}
+
 // Rows y in [YLO, YHI], z in [ZLO, ZHI] of a 4 x 4 x 2 register block:
 // acc[x + 4 (y + 4 z)] += wx[x] (wy[y] (wz[z] v)), weights as (w, w) pairs.
 template <int YLO, int YHI, int ZLO, int ZHI>
@@ -808,70 +876,11 @@ __global__ void __launch_bounds__(RegCfg<CPW, tap_rec(3, WM)>::NW * 32, RegCfg<C
     const int nvis = item_visits(it), vs = item_stride(it);
     const int nbat = (nvis + C::Batch - 1) / C::Batch;
     auto batch_size = [&](int bb) { return (nvis - bb + nbat - 1) / nbat; };
-    // issue the copies of batch bb into buffer buf.  A warp takes rounds of 32
-    // samples (warp, warp + NW, ... in units of 32): lane l resolves sample q0 + l
-    // (its sorted position and neighbour delta), then the warp copies the round's
-    // plan records and value rows in 16-byte pieces, consecutive lanes on
-    // consecutive pieces of a row
     auto issue = [&](int bb, int buf) {
         unsigned char *B = ub + buf * C::Buf;
-        float2 *rv = reinterpret_cast<float2 *>(B);
-        int *rr = reinterpret_cast<int *>(B + C::OffR);
-        int *rd = reinterpret_cast<int *>(B + C::OffD);
-        const int nb = batch_size(bb);
-        for (int q0 = warp * 32; q0 < nb; q0 += NW * 32) {
-            const int q = q0 + lane, nq = min(32, nb - q0);
-            int j = 0;
-            if (q < nb) {
-                // batch bb takes visits bb, bb + nbat, bb + 2 nbat, ...: every batch
-                // mixes the neighbour ranges, so all warps find work in it
-                const int v = it.v0 + (bb + q * nbat) * vs;
-                // range: the last one whose prefix is <= v (empty ranges share the
-                // prefix of the next one and are skipped)
-                int lo = 0, hi = NR;
-                while (hi - lo > 1) {
-                    const int m = (lo + hi) >> 1;
-                    if (s_pre[m] <= v) lo = m;
-                    else hi = m;
-                }
-                j = s_beg[lo] + (v - s_pre[lo]);
-                rd[q] = s_dlt[lo];
-            }
-            // plan records: REC / 4 pieces per sample.  Lanes past the round's last
-            // piece copy nothing (a zero-size copy still writes its destination)
-            constexpr int RP = REC / 4;
-            for (int e0 = 0; e0 < nq * RP; e0 += 32) {
-                const int e = e0 + lane;
-                const bool in = e < nq * RP;
-                const int sq = in ? e / RP : 0, part = e - sq * RP;
-                const int js = __shfl_sync(0xffffffffu, j, sq);
-                if (in) cp_async16(rr + (q0 + sq) * REC + 4 * part, P.wtap + (int64_t)js * REC + 4 * part, true);
-            }
-            // value rows: channels c0 .. c0 + CPW - 1, zero-filled past nch; lanes past
-            // the round's last piece copy nothing
-            if (nch % 2 == 0) {
-                constexpr int VP = CPW / 2;  // 16-byte pieces (two channels) per row
-                for (int e0 = 0; e0 < nq * VP; e0 += 32) {
-                    const int e = e0 + lane;
-                    const bool in = e < nq * VP;
-                    const int sq = in ? e / VP : 0, part = e - sq * VP;
-                    const int js = __shfl_sync(0xffffffffu, j, sq);
-                    const int ch = c0 + 2 * part;
-                    const bool ok = ch < nch;
-                    if (in) cp_async16(rv + (q0 + sq) * CPW + 2 * part, P.vals + (ok ? (int64_t)js * nch + ch : 0), ok);
-                }
-            } else {
-                for (int e0 = 0; e0 < nq * CPW; e0 += 32) {
-                    const int e = e0 + lane;
-                    const bool in = e < nq * CPW;
-                    const int sq = in ? e / CPW : 0, part = e - sq * CPW;
-                    const int js = __shfl_sync(0xffffffffu, j, sq);
-                    const int ch = c0 + part;
-                    const bool ok = ch < nch;
-                    if (in) cp_async8(rv + (q0 + sq) * CPW + part, P.vals + (ok ? (int64_t)js * nch + ch : 0), ok);
-                }
-            }
-        }
+        stage_samples<CPW, REC, NR, NW>(P, it, vs, bb, nbat, batch_size(bb), s_pre, s_beg, s_dlt, c0, warp, lane,
+                                        reinterpret_cast<float2 *>(B), reinterpret_cast<int *>(B + C::OffR),
+                                        reinterpret_cast<int *>(B + C::OffD));
     };
     // this lane's block (block id warp * G + group) and the warp's blocks' bits in the
     // sample masks
@@ -1053,15 +1062,14 @@ __device__ __forceinline__ void reg2_rows(float2 (&acc)[32], const float2 (&wx2)
 // occupancy mask holds x in bits 0..15 and y in bits 16..31.
 constexpr int kReg2Tile = 16;
 constexpr int kReg2Pts = kReg2Tile * kReg2Tile;
-template <int CPW>
+template <int CPW, int REC>
 struct Reg2Cfg {
     static constexpr int G = 32 / CPW;
     static constexpr int NW = 8 / G;
     static constexpr int MinBlocks = CPW == 32 ? 2 : (CPW == 16 ? 3 : 4);
     static constexpr int Batch = CPW == 32 ? 96 : (CPW == 16 ? 96 : 80);
-    static constexpr size_t OffW = (size_t)Batch * CPW * sizeof(float2);
-    static constexpr size_t OffX = OffW + (size_t)Batch * 16 * sizeof(float);
-    static constexpr size_t OffD = OffX + (size_t)Batch * 4 * sizeof(int);
+    static constexpr size_t OffR = (size_t)Batch * CPW * sizeof(float2);
+    static constexpr size_t OffD = OffR + (size_t)Batch * REC * sizeof(int);
     static constexpr size_t Buf = OffD + (size_t)Batch * sizeof(int);
     static constexpr size_t OffTW = 2 * Buf;
     static constexpr size_t OffM = OffTW + (size_t)Batch * 32 * sizeof(float2);
@@ -1073,12 +1081,11 @@ struct Reg2Cfg {
 };
 
 template <int WM, int CPW>
-__global__ void __launch_bounds__(Reg2Cfg<CPW>::NW * 32, Reg2Cfg<CPW>::MinBlocks)
+__global__ void __launch_bounds__(Reg2Cfg<CPW, tap_rec(2, WM)>::NW * 32, Reg2Cfg<CPW, tap_rec(2, WM)>::MinBlocks)
     spread_reg2_kernel(const SpreadIL P) {
-    using C = Reg2Cfg<CPW>;
+    constexpr int D = 2, DW = D * WM, REC = tap_rec(D, WM);
+    using C = Reg2Cfg<CPW, REC>;
     constexpr int G = C::G, NW = C::NW;
-    constexpr int D = 2, DW = D * WM;
-    static_assert(DW <= 16, "raw weights of one sample fit 16 entries");
     extern __shared__ __align__(16) unsigned char smraw[];
     int *s_pos = reinterpret_cast<int *>(smraw);
     unsigned char *ub = smraw + kReg2Pts * sizeof(int);
@@ -1091,7 +1098,7 @@ __global__ void __launch_bounds__(Reg2Cfg<CPW>::NW * 32, Reg2Cfg<CPW>::MinBlocks
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nch = P.ch.nch;
     const int cl = lane % CPW, grpl = lane / CPW;
-    const int c0 = blockIdx.y * CPW, c = c0 + cl;
+    const int c0 = blockIdx.y * CPW;
     int org[2], text[2], wrap[2];
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
@@ -1112,23 +1119,12 @@ __global__ void __launch_bounds__(Reg2Cfg<CPW>::NW * 32, Reg2Cfg<CPW>::MinBlocks
     const int nvis = item_visits(it), vs = item_stride(it);
     const int nbat = (nvis + C::Batch - 1) / C::Batch;
     auto batch_size = [&](int bb) { return (nvis - bb + nbat - 1) / nbat; };
+    // as spread_reg3_kernel's: a warp resolves and copies rounds of 32 samples
     auto issue = [&](int bb, int buf) {
         unsigned char *B = ub + buf * C::Buf;
-        float2 *rv = reinterpret_cast<float2 *>(B);
-        float *rw = reinterpret_cast<float *>(B + C::OffW);
-        int *rx = reinterpret_cast<int *>(B + C::OffX);
-        int *rd = reinterpret_cast<int *>(B + C::OffD);
-        const int nb = batch_size(bb);
-        for (int q = warp; q < nb; q += NW) {
-            const int v = it.v0 + (bb + q * nbat) * vs;  // batches mix the neighbour ranges
-            const unsigned le = __ballot_sync(0xffffffffu, lane < NR && s_pre[lane] <= v);
-            const int r = 31 - __clz(le);
-            const int64_t j = (int64_t)s_beg[r] + (v - s_pre[r]);
-            if (lane < CPW) cp_async8(rv + q * CPW + lane, P.vals + j * nch + (c < nch ? c : 0), c < nch);
-            if (lane < DW) cp_async4(rw + q * 16 + lane, P.wtap + j * tap_rec(D, WM) + lane);
-            if (lane < D) cp_async4(rx + q * 4 + lane, P.xtap + j * tap_rec(D, WM) + lane);
-            if (lane == 0) rd[q] = s_dlt[r];
-        }
+        stage_samples<CPW, REC, NR, NW>(P, it, vs, bb, nbat, batch_size(bb), s_pre, s_beg, s_dlt, c0, warp, lane,
+                                        reinterpret_cast<float2 *>(B), reinterpret_cast<int *>(B + C::OffR),
+                                        reinterpret_cast<int *>(B + C::OffD));
     };
     // this lane's block: bid = warp * G + group, 4 blocks along x, 2 along y
     const int bid = warp * G + grpl;
@@ -1160,19 +1156,19 @@ __global__ void __launch_bounds__(Reg2Cfg<CPW>::NW * 32, Reg2Cfg<CPW>::MinBlocks
         cp_async_commit();
         unsigned char *B = ub + cur * C::Buf;
         const float2 *rv = reinterpret_cast<const float2 *>(B);
-        const float *rw = reinterpret_cast<const float *>(B + C::OffW);
-        const int *rx = reinterpret_cast<const int *>(B + C::OffX);
+        const float *rw = reinterpret_cast<const float *>(B + C::OffR);  // records: weights, then first taps
+        const int *rx = reinterpret_cast<const int *>(B + C::OffR) + DW;
         const int *rd = reinterpret_cast<const int *>(B + C::OffD);
         float2 *tw = reinterpret_cast<float2 *>(ub + C::OffTW);
         unsigned *tm = reinterpret_cast<unsigned *>(ub + C::OffM);
         const int nb = batch_size(b);
         for (int q = warp; q < nb; q += NW) {
             float wv = 0.f;
-            int d = rx[q * 4 + la] - orga;
+            int d = rx[q * REC + la] - orga;
             if (((rd[q] >> la) & 1) && d >= 0) d -= nosa;
             int i = lt - d;
             if (wrapa && i < 0) i += wrapa;
-            if (lt < texta && i >= 0 && i < wa) wv = rw[q * 16 + la * WM + i];
+            if (lt < texta && i >= 0 && i < wa) wv = rw[q * REC + la * WM + i];
             tw[q * 32 + lane] = make_float2(wv, wv);
             const unsigned m = __ballot_sync(0xffffffffu, wv != 0.f);
             if (lane == 0) tm[q] = m;
@@ -1330,7 +1326,7 @@ int launch_spread_reg3_t(const SpreadIL &P, int nitems, int nchunks, cudaStream_
 
 template <int WM, int CPW>
 int launch_spread_reg2_t(const SpreadIL &P, int nitems, int nchunks, cudaStream_t s) {
-    using C = Reg2Cfg<CPW>;
+    using C = Reg2Cfg<CPW, tap_rec(2, WM)>;
     auto k = spread_reg2_kernel<WM, CPW>;
     PFB_RAISE_SMEM(k, (int)C::Smem);
     dim3 grid(nitems, nchunks);
