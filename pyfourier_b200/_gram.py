@@ -239,11 +239,10 @@ def _gram_core(gm: GramMatrix, x):
     n = ctypes.c_size_t()
     _lib.check(L.pfb_gram_workspace_size(h.handle, B, ctypes.byref(n)))
     ws = torch.empty(int(n.value), dtype=torch.uint8, device=gm.device)
-    st = ctypes.c_void_p(torch.cuda.current_stream(gm.device).cuda_stream)
+    st = torch.cuda.current_stream(gm.device).cuda_stream
     zs = gm.zmap_s_kernel
-    zp = ctypes.c_void_p(zs.data_ptr()) if zs is not None else None
-    _lib.check(L.pfb_gram_apply(h.handle, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()), B,
-                                zp, ctypes.c_void_p(ws.data_ptr()), ws.numel(), st))
+    zp = zs.data_ptr() if zs is not None else None
+    _lib.check(L.pfb_gram_apply(h.handle, x.data_ptr(), out.data_ptr(), B, zp, ws.data_ptr(), ws.numel(), st))
     return out
 
 
@@ -287,10 +286,10 @@ def sparse_gram(image, gram_matrix, norm=None, device="cpu", threadsperblock=128
     batch_shape = xc.shape[: xc.ndim - nd - (1 if has_c else 0)]
     if has_c and xc.shape[-nd - 1] != C:
         raise ValueError(f"image needs an axis of size {C} before the spatial axes")
-    B = int(np.prod(batch_shape)) if len(batch_shape) else 1
+    B = math.prod(batch_shape)
     y = SparseGramFunction.apply(xc.reshape(B, C, *gm.image_shape), gm)
     y = y.reshape(xc.shape)
-    if not torch.is_complex(torch.empty((), dtype=dtype)):
+    if not dtype.is_complex:
         y = y.real
     y = to_caller(y, idevice, dtype)
     return y.detach().numpy() if as_numpy else y

@@ -30,11 +30,11 @@ def norm_code(norm):
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    return torch.cuda.current_stream(dev).cuda_stream
 
 
 class _Ctx:
@@ -49,7 +49,7 @@ class _Ctx:
         self.norm = norm
         self.nframes = self.interp.nframes
         self.C = basis.shape[1] if basis is not None else self.nframes
-        self.G = float(np.prod(plan.os_shape))
+        self.G = float(math.prod(plan.os_shape))
         s = self.interp.scale
         self.fac_fwd = (1.0 / s) / (math.sqrt(self.G) if norm == _lib.PFB_NORM_ORTHO else 1.0)
         self.fac_adj = (1.0 / s) / (math.sqrt(self.G) if norm == _lib.PFB_NORM_ORTHO else self.G)
@@ -66,22 +66,16 @@ class _Ctx:
             yield start, min(Lseg, start + step)
 
     def opts(self, batch, seg, flags=0):
-        o = _lib.ApplyT()
-        o.batch = int(batch)
-        o.ncoeff = int(self.C)
-        o.basis = self.basis.data_ptr() if self.basis is not None else None
-        o.weight = self.weight.data_ptr() if self.weight is not None else None
+        basis = self.basis.data_ptr() if self.basis is not None else None
+        weight = self.weight.data_ptr() if self.weight is not None else None
         p = self.plan
+        nseg, b0_time, b0_space = 1, None, None
         if p.zmap_s_kernel is not None:
             start, stop = seg
-            o.nseg = stop - start
-            o.b0_time = p.zmap_t_kernel[start:stop].data_ptr()
-            o.b0_space = p.zmap_s_kernel[start:stop].data_ptr()
-        else:
-            o.nseg = 1
-        o.norm = self.norm
-        o.flags = flags
-        return o
+            nseg = stop - start
+            b0_time = p.zmap_t_kernel[start:stop].data_ptr()
+            b0_space = p.zmap_s_kernel[start:stop].data_ptr()
+        return _lib.ApplyT(batch, self.C, nseg, basis, weight, b0_time, b0_space, self.norm, flags)
 
     def workspace(self, opts):
         """Workspace of the fastest path for these apply options (caching allocator)."""
@@ -140,8 +134,7 @@ def traj_grad_core(ctx: _Ctx, image_side, values, factor):
         o = ctx.opts(B, seg, _lib.PFB_FLAG_ACCUMULATE)
         ws = ctx.workspace(o)
         _lib.check(L.pfb_nufft_traj_grad(ctx.interp.handle, ctypes.byref(o), _ptr(image_side), _ptr(values),
-                                         ctypes.c_void_p(grad.data_ptr()), ctypes.c_float(factor), _ptr(ws),
-                                         ws.numel(), st))
+                                         _ptr(grad), factor, _ptr(ws), ws.numel(), st))
     return grad
 
 
@@ -223,6 +216,8 @@ def _split_weight(weight, sample_shape, dev):
         return None, None
     w = _as_tensor(weight)
     w = w.to(dev)
+    if w.dtype == torch.float32 and w.shape == sample_shape and w.is_contiguous():
+        return w.reshape(-1), None
     if not torch.is_complex(w):
         w = w.to(torch.float32)
         lead = w.ndim - len(sample_shape)
@@ -240,6 +235,8 @@ def _split_weight(weight, sample_shape, dev):
 
 def _to_compute(x, dev):
     x = _as_tensor(x)
+    if x.dtype == torch.complex64 and x.device == dev:
+        return x, x
     if x.dtype in (torch.float16, torch.float32, torch.float64, torch.bfloat16):
         xc = x.to(dev, torch.float32).to(torch.complex64)
     else:
@@ -248,7 +245,7 @@ def _to_compute(x, dev):
 
 
 def _finish(out, dtype, idevice, as_numpy):
-    if not torch.is_complex(torch.empty((), dtype=dtype)):
+    if not dtype.is_complex:
         out = out.real
     out = to_caller(out, idevice, dtype)
     return out.detach().numpy() if as_numpy else out
@@ -370,7 +367,7 @@ def nufft(image, coord=None, shape=None, nufft_plan=None, basis=None, zmap=None,
     if has_c and (x.ndim < nd + 1 or x.shape[-nd - 1] != C):
         raise ValueError(f"image needs a contrast/coefficient axis of size {C} before the spatial axes")
     batch_shape = x.shape[: x.ndim - nd - (1 if has_c else 0)]
-    B = int(np.prod(batch_shape)) if len(batch_shape) else 1
+    B = math.prod(batch_shape)
     sshape = _sample_shape(ip)
     wps, wfull = _split_weight(weight, sshape, dev)
     ctx = _Ctx(plan, basis_t, wps, norm_code(norm))
@@ -421,7 +418,7 @@ def nufft_adj(kspace, coord=None, shape=None, nufft_plan=None, basis=None, zmap=
     if tuple(k.shape[k.ndim - len(sshape):]) != tuple(sshape):
         raise ValueError(f"k-space trailing shape {tuple(k.shape[k.ndim - len(sshape):])} != {sshape}")
     batch_shape = k.shape[: k.ndim - len(sshape)]
-    B = int(np.prod(batch_shape)) if len(batch_shape) else 1
+    B = math.prod(batch_shape)
     wps, wfull = _split_weight(weight, sshape, dev)
     ctx = _Ctx(plan, basis_t, wps, norm_code(norm))
     if host and B >= 2 and wfull is None:

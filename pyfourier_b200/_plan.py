@@ -41,14 +41,20 @@ def resolve_device(device, fallback=None):
     default) and ``None`` select ``fallback`` when it is a CUDA device, else the
     current CUDA device; results are returned on the caller's device.
     """
-    if not torch.cuda.is_available():
+    # a tensor or a plan on a GPU: CUDA runs, and asking the driver again costs 3 us
+    on_gpu = isinstance(fallback, torch.device) and fallback.type == "cuda"
+    if not on_gpu and not torch.cuda.is_available():
         raise RuntimeError("pyfourier_b200 needs a CUDA device (no CPU fallback)")
     if isinstance(device, torch.device):
+        if device.type == "cuda" and device.index is not None:
+            return device
         device = str(device)
     if isinstance(device, str) and device.startswith("cuda"):
         return torch.device(device if ":" in device else f"cuda:{torch.cuda.current_device()}")
     if isinstance(device, int) and device >= 0:
         return torch.device(f"cuda:{device}")
+    if on_gpu:
+        return fallback
     if fallback is not None and torch.device(fallback).type == "cuda":
         return torch.device(fallback)
     return torch.device(f"cuda:{torch.cuda.current_device()}")
