@@ -146,6 +146,7 @@ struct FftAxis {
     int ns[kFftMaxStages] = {};
     int twoff[kFftMaxStages] = {};
     int rootoff[kFftMaxStages] = {};
+    int swapoff = 0;  // rows of two stages: the twiddles of the two radices in the other order
     unsigned magic[kFftMaxStages] = {};    // floor(i / ns) = umulhi(i, magic) for i < 2^16 (ns > 1)
     unsigned magic_m[kFftMaxStages] = {};  // the same for n / radix
     const float2 *tw = nullptr;

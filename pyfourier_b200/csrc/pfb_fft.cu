@@ -179,6 +179,11 @@ bool make_axis(int n, bool rows, FftAxis *fa, std::vector<float2> &tw, size_t *b
         }
         ns *= r;
     }
+    if (rows && fa->nst == 2) {  // see gram_two
+        fa->swapoff = (int)(tw.size() - *base);
+        for (int q = 1; q < rad[0]; ++q)
+            for (int j = 0; j < rad[1]; ++j) root((double)j * q, (double)n);
+    }
     return true;
 }
 

@@ -73,3 +73,13 @@ def test_elementwise_planes(B, F):
 @pytest.mark.parametrize("K, L", [(0, 0), (3, 0), (0, 2), (4, 3)])
 def test_grids_and_segments(n, os, K, L):
     _check(n, os, 3, K=K, L=L)
+
+
+# (n, embedded length) of the rows: two stages with constants, alike and unlike, with radices
+# to 16 and above, odd, dense and single-point images
+@pytest.mark.parametrize("n, os", [(48, 96), (97, 160), (128, 256), (1, 240), (100, 200), (125, 250), (176, 352),
+                                   (256, 512), (150, 150), (144, 144)])
+@pytest.mark.parametrize("B, F", [(1, 1), (9, 1), (2, 3)])
+def test_elementwise_rows_of_two_stages(n, os, B, F):
+    _check((5, n), (10, os), B, F=F)
+    _check((2, 3, n), (4, 6, os), B, F=F)
