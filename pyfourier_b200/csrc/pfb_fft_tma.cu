@@ -16,7 +16,8 @@ constexpr int kCols = 16;                 // vectors per CTA
 constexpr int kThreads = 256;
 constexpr int kPairStreams = kThreads / (kCols / 2);  // butterflies: a thread takes 2 columns
 
-// at most 256: a tile's rows are one box
+// at most 256 (kTmaMax): a tile's rows are one box
+constexpr int kTmaMax = 256;
 constexpr bool tma_length(int n) { return n == 250 || n == 240 || n == 160 || n == 256; }
 struct StagePlan {
     int radix[2];
@@ -169,7 +170,7 @@ struct ColTma {
     int C;
     int64_t nvol;
     const float *apod_ax, *apod_mid, *apod_x;
-    const float2 *Cl;       // B0 segment factors on the image side (nseg x nvol), or null
+    const float2 *Cl;       // B0 segment factors on the image side (nseg x nvol), in the SEG form
     float factor;
     int accumulate;
     int *err;               // set to 1 when a wait gives up (the results are then invalid)
@@ -226,7 +227,10 @@ struct TileInfo {
 // src_map: the pass's source as 4D (2X floats, rows, mid, source plane).
 // Two ring slots (the next tile loads while this one transforms; 2 CTAs per SM): one slot
 // and 3 CTAs per SM took 1.30 against 1.21 ms for the 200^3 z pass.
-// SEG: B0 factors and segment sums; the plain instantiation keeps its simpler loops.
+// SEG: B0 factors and segment sums; the plain instantiation keeps its simpler loops.  The
+// segments are summed in registers (added to the image one by one, 192^2 x 768 with 8
+// segments of 240 points took 1072 us against 897; the factor loads have to be ahead of the
+// products, 4 rows at a time: row by row 1418 us).
 template <bool SEG>
 __global__ void __launch_bounds__(kThreads, 2)
     col_tma_kernel(const __grid_constant__ CUtensorMap src_map, const ColTma P) {
@@ -272,6 +276,10 @@ __global__ void __launch_bounds__(kThreads, 2)
             if (t < P.ntiles) issue(t, l, s);
         }
     }
+    constexpr int kRows = SEG ? kTmaMax / NS : 1;  // rows of a column pair that a thread writes
+    float4 sum[kRows];
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int k = 0;; ++k) {
         int lk;
         const int t = block_of(k, lk);
@@ -310,55 +318,57 @@ __global__ void __launch_bounds__(kThreads, 2)
         // forward transform's position (n - pp) mod n
         const int64_t obase = (int64_t)ti.plane * P.nvol + (int64_t)ti.mid * P.out_mid;
         if (SEG) {
-            // kU rows per thread at a time: the factor and partial-sum loads of an
-            // adjoint last pass are all in flight before the first product
-            constexpr int kU = 3;
-            const bool seg_sum = P.accumulate || ti.l > 0;
-            const float2 *clp =
-                P.Cl ? P.Cl + (int64_t)ti.l * P.nvol + (int64_t)ti.mid * P.out_mid : nullptr;
-            for (int o0 = stream; o0 < P.lout; o0 += kU * NS) {
-                float4 cc[kU], old[kU];
-                float aa[kU];
+            // the segments of the block are summed in registers: kRows rows of two columns
+            const float2 *clp = P.Cl + (int64_t)ti.l * P.nvol + (int64_t)ti.mid * P.out_mid + xs;
+            // kU rows at a time: their factor loads are in flight before the first product
+            constexpr int kU = 4;
+#pragma unroll
+            for (int u0 = 0; u0 < kRows; u0 += kU) {
+                float4 cc[kU];
 #pragma unroll
                 for (int u = 0; u < kU; ++u) {
-                    const int o = o0 + u * NS;
-                    const int oc = o < P.lout ? o : 0;
-                    if (xin) {
-                        const int64_t off = (int64_t)oc * P.out_ax + x;
-                        cc[u] = clp ? __ldg(reinterpret_cast<const float4 *>(clp + off))
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-                        // segments after the first add to the sum this thread stored for
-                        // the ones before (same addresses, same thread: a plain load)
-                        old[u] = seg_sum ? *reinterpret_cast<const float4 *>(P.dst + obase + off)
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-                        aa[u] = P.apod_ax ? P.apod_ax[oc] : 1.f;
-                    }
+                    const int o = min(stream + (u0 + u) * NS, P.lout - 1);
+                    cc[u] = __ldg(reinterpret_cast<const float4 *>(clp + (int64_t)o * P.out_ax));
                 }
 #pragma unroll
                 for (int u = 0; u < kU; ++u) {
-                    const int o = o0 + u * NS;
-                    if (o >= P.lout || !xin) continue;
+                    const int o = min(stream + (u0 + u) * NS, P.lout - 1);
                     int pp = o - P.hn;
                     if (pp < 0) pp += n;
                     const int q = pp == 0 ? 0 : n - pp;
-                    float4 w = *reinterpret_cast<const float4 *>(R + q * kTmaPitch + col);
-                    if (clp) {  // times conj(C_l) of the tile's segment
-                        const float2 v0 = cmulc(make_float2(w.x, w.y), make_float2(cc[u].x, cc[u].y));
-                        const float2 v1 = cmulc(make_float2(w.z, w.w), make_float2(cc[u].z, cc[u].w));
-                        w = make_float4(v0.x, v0.y, v1.x, v1.y);
-                    }
-                    const float a0 = aa[u] * amid0, a1 = aa[u] * amid1;
+                    const float4 w = *reinterpret_cast<const float4 *>(R + q * kTmaPitch + col);
+                    // times conj(C_l) of the tile's segment
+                    const float2 v0 = cmulc(make_float2(w.x, w.y), make_float2(cc[u].x, cc[u].y));
+                    const float2 v1 = cmulc(make_float2(w.z, w.w), make_float2(cc[u].z, cc[u].w));
+                    float4 &t = sum[u0 + u];
+                    t.x += v0.x;
+                    t.y += v0.y;
+                    t.z += v1.x;
+                    t.w += v1.y;
+                }
+            }
+            if (ti.l + 1 == P.nseg) {
+#pragma unroll
+                for (int u = 0; u < kRows; ++u) {
+                    const int o = stream + u * NS;
+                    float4 w = sum[u];
+                    sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (o >= P.lout || !xin) continue;
+                    const float a = P.apod_ax ? P.apod_ax[o] : 1.f;
+                    const float a0 = a * amid0, a1 = a * amid1;
+                    float4 *d = reinterpret_cast<float4 *>(P.dst + obase + (int64_t)o * P.out_ax + x);
                     w.x *= a0;
                     w.y *= a0;
                     w.z *= a1;
                     w.w *= a1;
-                    if (seg_sum) {
-                        w.x += old[u].x;
-                        w.y += old[u].y;
-                        w.z += old[u].z;
-                        w.w += old[u].w;
+                    if (P.accumulate) {
+                        const float4 old = *d;
+                        w.x += old.x;
+                        w.y += old.y;
+                        w.z += old.z;
+                        w.w += old.w;
                     }
-                    *reinterpret_cast<float4 *>(P.dst + obase + (int64_t)o * P.out_ax + x) = w;
+                    *d = w;
                 }
             }
         } else {
@@ -549,7 +559,7 @@ bool encode_col_map(CUtensorMap *m, const void *base, int X, int rows, int nmid,
 // with 64):
 //              250          240          160        256
 //   x fwd      1477 / 2052  922 / 1110   407 / 432  674 / 763    here
-//   image out  1178 / 1262  1150 / 1536  303 / 270  5.8 / 6.4    here but 160
+//   image out  1178 / 1262   897 / 1536  303 / 270  5.8 / 6.4    here but 160
 //   image in   1114 / 1067  1278 / 858   330 / 280               direct
 //   y fwd      1117 / 1111               307 / 286               direct
 //   y inv      1231 / 1079               326 / 260               direct
@@ -588,7 +598,7 @@ int launch_col_tma(const ColPass &P, int pass, cudaStream_t s) {
     auto a16 = [](const void *q) { return ((uintptr_t)q & 15u) == 0; };
     if (!a16(P.src) || !a16(P.dst)) return 0;
     if (P.Cl && !a16(P.Cl)) return 0;
-    if (P.ch.L < 1) return 0;
+    if (P.ch.L < 1 || (P.ch.L > 1 && !P.Cl)) return 0;
     for (int64_t v : {P.in_ax, P.in_mid, P.in_plane, P.out_ax, P.out_mid, P.nvol})
         if (v % 2 != 0) return 0;
     ColTma T{};
@@ -620,7 +630,7 @@ int launch_col_tma(const ColPass &P, int pass, cudaStream_t s) {
                         n))
         return 0;
     const size_t smem = (size_t)3 * n * kTmaPitch * sizeof(float2);
-    auto kern = P.Cl || T.nseg > 1 ? col_tma_kernel<true> : col_tma_kernel<false>;
+    auto kern = P.Cl ? col_tma_kernel<true> : col_tma_kernel<false>;
     PFB_RAISE_SMEM(kern, (int)smem);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
