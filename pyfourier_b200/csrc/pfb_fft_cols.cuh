@@ -74,22 +74,26 @@ struct ColStoreImage {
     const float *apod;  // null: no deapodisation
     float a;
     bool accumulate;
-    const float2 *cl;   // null: no B0 factors
+    const float2 *cl;   // SEG: the segment's factors
     float2 *acc;        // this column's partial sums, pitch `pitch`
     int pitch;
     bool first, last;
     __device__ __forceinline__ void operator()(int k, float2 v) const {
         const int o = wrap(wrap(n - k, n) + hn, n);
-        if (o >= lout || !on) return;
+        const bool in = o < lout && on;
+        // the factors first and without a branch, so that those of a butterfly are in flight
+        // together
+        const int oc = o < lout ? o : 0;
+        const float f = apod ? a * __ldg(apod + oc) : a;
+        if (SEG) v = cmulc(v, __ldg(step(cl, oc, bytes)));
+        if (!in) return;
         if (SEG) {
-            if (cl) v = cmulc(v, __ldg(step(cl, o, bytes)));
             if (!first) v = cadd(v, acc[o * pitch]);
             if (!last) {
                 acc[o * pitch] = v;
                 return;
             }
         }
-        const float f = apod ? a * __ldg(apod + o) : a;
         v = make_float2(v.x * f, v.y * f);
         float2 *d = step(dst, o, bytes);
         if (accumulate) v = cadd(v, *d);
@@ -148,7 +152,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) col_kernel(const
         float2 *dst = P.dst + (int64_t)plane * P.nvol + off + x;
         const float2 *src = P.src + (int64_t)grp * P.ch.nch * P.in_plane + (int64_t)mid * P.in_mid + xs;
         auto chan = [&](int l) { return P.ch.K ? (l * P.ch.B + b) * Kc + c : l * P.ch.B + b; };
-        if (P.ch.L == 1 && !P.Cl) {
+        if (!P.Cl) {  // one segment
             ColLoad<false> ld{src + chan(0) * P.in_plane, (int)P.in_ax * 8, n, hn, P.lin};
             ColStoreImage<false> st{dst, (int)P.out_ax * 8, n, hn, P.lout, xin, P.apod_ax, a, P.accumulate != 0};
             run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
@@ -158,7 +162,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) col_kernel(const
         for (int l = 0; l < P.ch.L; ++l) {
             ColLoad<false> ld{src + chan(l) * P.in_plane, (int)P.in_ax * 8, n, hn, P.lin};
             ColStoreImage<true> st{dst, (int)P.out_ax * 8, n, hn, P.lout, xin, P.apod_ax, a, P.accumulate != 0,
-                                   P.Cl ? P.Cl + (int64_t)l * P.nvol + off + xs : nullptr, acc, NV, l == 0,
+                                   P.Cl + (int64_t)l * P.nvol + off + xs, acc, NV, l == 0,
                                    l + 1 == P.ch.L};
             if (l > 0) __syncthreads();  // the previous segment's last stage has read its buffer
             run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
@@ -177,7 +181,7 @@ int launch_nv(ColPass P, cudaStream_t s) {
     P.dk = Div(P.ch.K);
     P.db = Div(P.ch.B);
     P.dc = Div(P.C);
-    const int bufs = (P.fa.nst > 2 ? 2 : 1) + (MODE == kImageOut && (P.ch.L > 1 || P.Cl) ? 1 : 0);
+    const int bufs = (P.fa.nst > 2 ? 2 : 1) + (MODE == kImageOut && P.Cl ? 1 : 0);
     const size_t smem = (size_t)bufs * ColAddr<NV>::size(P.fa.n) * sizeof(float2);
     auto k = col_kernel<MODE, NV, BIG>;
     PFB_RAISE_SMEM(k, (int)smem);
