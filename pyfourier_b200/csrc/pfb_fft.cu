@@ -17,7 +17,7 @@
 // written, so a forward transform of an N^3 image onto an n^3 grid moves about
 // N^3 + 2 n N^2 + 2 n^2 N + n^3 elements per plane instead of the 2 n^3 per pass
 // of an unpruned transform, and the pad, crop and channel transpose cost nothing
-// extra.  The passes' kernels are in pfb_fft_cols.cu and pfb_fft_rows.cu.
+// extra.  The passes' kernels: pfb_fft_cols.cuh, pfb_fft_rows.cu, pfb_fft_tma.cu.
 #include <cmath>
 #include <vector>
 

@@ -4,7 +4,7 @@
 // after the other; out[v] = T[v] @ in[v] is the evident intent of _bmatvec/_bdot.py:16-115).
 //
 // The embedding's shift does not change a product with a function of frequency, so the
-// image sits at the grid's origin: the outer axes' passes (pfb_fft_cols.cu) and this one
+// image sits at the grid's origin: the outer axes' passes (pfb_fft_cols.cuh) and this one
 // read N rows and zero-pad them, and write back N rows; no grid of the full size exists
 // and pad, crop and product cost no pass of their own.  A CTA holds V vectors of one grid
 // row: all K planes of `nbv` batch items (or, for the elementwise kernel, V batch items of
