@@ -532,7 +532,9 @@ int pfb_gram_create(int ndim, const int *shape, const int *os_shape, int ncoeff,
         delete g;
         return fail(PFB_ERR_CUDA, std::string("kernel copy: ") + cudaGetErrorString(e));
     }
-    if (ndim >= 2) g->fused = fft_axes(ndim, g->nos, g->ax, &g->d_tw);
+    bool dense = nseg == 1;  // the grid is the image: no pad and crop to save
+    for (int a = 0; a < ndim; ++a) dense = dense && g->n[a] == g->nos[a];
+    if (ndim >= 2) g->fused = fft_axes(ndim, g->nos, dense, g->ax, &g->d_tw);
     *out = g;
     return PFB_OK;
 }

@@ -433,8 +433,9 @@ int counting_sort_pairs(const int *keys, const int *vals, int *keys_out, int *va
                         void *temp, size_t temp_bytes, cudaStream_t s);
 
 // fused pruned FFT (pfb_fft.cu).  The Gram: 1 and the axes with a device twiddle table
-// (pool memory of the current device) when every axis is taken, else 0.
-int fft_axes(int ndim, const int *nos, FftAxis *ax, float2 **d_tw);
+// (pool memory of the current device) when every axis is taken, else 0; dense: a Gram whose
+// grid is the image.
+int fft_axes(int ndim, const int *nos, bool dense, FftAxis *ax, float2 **d_tw);
 // Gram apply: images [plane][*n] -> out through grids of N rows (see pfb_fft_gram.cu);
 // planes = segments x batch x K; ws: gram_fused_workspace bytes
 struct GramFused {

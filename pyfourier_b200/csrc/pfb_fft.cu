@@ -189,7 +189,30 @@ bool make_axis(int n, bool rows, FftAxis *fa, std::vector<float2> &tw, size_t *b
 
 }  // namespace
 
-int fft_axes(int ndim, const int *nos, FftAxis *ax, float2 **d_tw) {
+// Where the prime stages lose to the library's transform (measured, us, library / here):
+// an axis that is itself a prime, with no part to spread over the first and last stage, when
+// two axes of a 3D grid are (16 planes of 61^3 454 / 509, 107^3 2908 / 3538, 96 x 107 x 107
+// 2100 / 2315; with one, 96 x 96 x 107, 1426 / 1290, with two of 37 245 / 233); and on the
+// dense Gram's grids, which the library transforms in place without pad and crop (128 planes
+// of 97^2 124 / 179, 127^2 224 / 252, 254^2 969 / 1043; 166^2 350 / 349, 123^2 163 / 120).
+// The 3D figures are of grids without oversampling; at 1.25, where the passes prune, the two
+// come out within 5 % (107^3, 8 coils, 1402 / 1475, 127^3 2565 / 2510).
+static bool prime_axes_lose(int ndim, const int *nos, bool dense) {
+    int bare = 0;
+    for (int a = 0; a < ndim; ++a) {
+        int m = nos[a], p = 1;  // the largest prime factor
+        for (int d = 2; m > 1; ++d)
+            while (m % d == 0) {
+                m /= d;
+                p = d;
+            }
+        if (dense && (p > 96 || (p > 32 && p == nos[a]))) return true;
+        if (p > 48 && p == nos[a]) ++bare;
+    }
+    return ndim == 3 && bare >= 2;
+}
+
+int fft_axes(int ndim, const int *nos, bool dense, FftAxis *ax, float2 **d_tw) {
     *d_tw = nullptr;
     int large = 0;  // axes with a prime factor above kMaxPrime
     for (int a = 0; a < ndim; ++a) {
@@ -198,7 +221,7 @@ int fft_axes(int ndim, const int *nos, FftAxis *ax, float2 **d_tw) {
         for (int r : rad)
             if (r > kMaxPrime) ++large;
     }
-    if (large > (ndim == 3 ? 1 : 0)) return 0;
+    if (large > (ndim == 3 ? 1 : 0) || prime_axes_lose(ndim, nos, dense)) return 0;
     std::vector<float2> tw;
     size_t base[3] = {0, 0, 0};
     for (int a = 0; a < ndim; ++a)
@@ -218,7 +241,7 @@ int fft_fused_ready(pfb_plan *p) {
     std::lock_guard<std::mutex> lk(p->fft_mu);
     if (p->fft_fused >= 0) return p->fft_fused;
     p->fft_fused = 0;
-    if (p->g.ndim < 2 || !fft_axes(p->g.ndim, p->g.nos, p->fft_ax, &p->d_fft_tw)) return 0;
+    if (p->g.ndim < 2 || !fft_axes(p->g.ndim, p->g.nos, false, p->fft_ax, &p->d_fft_tw)) return 0;
     // the TMA passes' flag and persistent grid (optional: without them the direct passes run)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

@@ -36,6 +36,11 @@ def _check(shape, B):
     assert float(torch.linalg.norm(y - ref) / torch.linalg.norm(ref)) < 2e-6
 
 
+@pytest.mark.parametrize("shape", [(47, 53, 10), (53, 10, 53), (10, 53, 59), (53, 53, 53), (53, 106, 10)])
+def test_several_prime_axes(shape):
+    _check(shape, 3)
+
+
 @pytest.mark.parametrize("n", LENGTHS)
 def test_each_axis(n):
     _check((n, 10), 3)

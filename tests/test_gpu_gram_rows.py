@@ -66,6 +66,12 @@ def test_elementwise_planes(B, F):
     _check((7, 12, 16), (14, 24, 32), B, F=F)
 
 
+@pytest.mark.parametrize("n", [(31, 37), (29, 31), (97, 20), (12, 194), (20, 178), (10, 41, 12)])
+@pytest.mark.parametrize("K, L", [(0, 0), (3, 0), (0, 2)])
+def test_dense_grids_with_prime_factors(n, K, L):
+    _check(n, n, 3, K=K, L=L)
+
+
 @pytest.mark.parametrize("n, os", [((16, 30), (16, 30)), ((16, 30), (32, 30)), ((9, 125), (9, 250)), ((1, 40), (1, 80)),
                                    ((62, 31), (124, 62)), ((27, 216), (54, 432)), ((8, 9, 10), (8, 9, 10)),
                                    ((6, 14, 22), (12, 14, 44)), ((10, 11, 53), (20, 22, 106)), ((6, 520), (12, 1040)),
