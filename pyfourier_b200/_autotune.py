@@ -90,7 +90,7 @@ def apply_choice(plan, tile, chunk):
 def autotune(plan, batch=1, basis=None, iters=3, tiles=None, chunks=None, use_cache=True):
     """Tune `plan` in place for `batch` coils (and `basis`, if given) and return
     the chosen ``{"tile": ..., "chunk": ..., "ms": ...}``."""
-    from ._nufft import _Ctx, adj_core, fwd_core
+    from ._nufft import _Ctx, _prep_basis, adj_core, fwd_core
 
     ip = plan.interpolator
     C = basis.shape[1] if basis is not None else ip.nframes
@@ -111,7 +111,7 @@ def autotune(plan, batch=1, basis=None, iters=3, tiles=None, chunks=None, use_ca
                       torch.randn(batch, C, *plan.shape, generator=g)).to(dev)
     y = torch.complex(torch.randn(batch, ip.total_samples, generator=g),
                       torch.randn(batch, ip.total_samples, generator=g)).to(dev)
-    bas = basis.to(dev, torch.complex64).contiguous() if basis is not None else None
+    bas = _prep_basis(basis, dev)
     best = None
     for tile in tiles:
         try:

@@ -29,7 +29,7 @@ import torch
 
 from ._b0 import mri_exp_approx
 from ._gram import GramMatrix, sparse_gram
-from ._plan import _as_tensor, resolve_device
+from ._plan import _as_tensor, dense, resolve_device
 
 
 def _dense_kernel(m, shape, basis, zmap, T, L, nbins):
@@ -59,7 +59,7 @@ def _dense_kernel(m, shape, basis, zmap, T, L, nbins):
         tu, inv = np.unique(t, return_inverse=True)  # fit over the distinct sampling times
         bt, zs = mri_exp_approx(_as_tensor(zmap).to(dev), tu, L, nbins, acorr=True)
         wl = torch.as_tensor(bt[:, inv], dtype=torch.complex64, device=dev).reshape(L, *m.shape)
-        zs = zs.to(torch.complex64).contiguous()
+        zs = dense(zs.to(torch.complex64))
     else:
         wl = torch.ones((1, *m.shape), dtype=torch.complex64, device=dev)
     mw = wl * m[None].to(torch.complex64)  # (L, nt, ny, nx)

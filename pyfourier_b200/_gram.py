@@ -31,7 +31,7 @@ import torch
 
 from . import _lib
 from ._b0 import mri_exp_approx
-from ._plan import _as_tensor, plan_nufft, resolve_device, to_caller
+from ._plan import _as_tensor, dense, plan_nufft, resolve_device, to_caller
 
 
 class _GramHandle:
@@ -39,7 +39,7 @@ class _GramHandle:
         L = _lib.load()
         self.device = torch.device(device)
         h = ctypes.c_void_p()
-        k = kernel.to(self.device, torch.complex64).contiguous()
+        k = dense(kernel.to(self.device, torch.complex64))
         with torch.cuda.device(self.device):
             s = torch.cuda.current_stream(self.device)
             _lib.check(L.pfb_gram_create(ndim, _lib.int_array(shape), _lib.int_array(os_shape), int(ncoeff),
@@ -137,7 +137,7 @@ def _psf_f64(vals, pplan, os_shape, basis):
     it = pplan.interpolator
     Ls = vals.shape[0]
     grid = torch.zeros((Ls, it.nframes, *pplan.os_shape), dtype=torch.complex128, device=dev)
-    v = vals.to(dev, torch.complex128).contiguous()
+    v = dense(vals.to(dev, torch.complex128))
     with torch.cuda.device(dev):
         st = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         _lib.check(_lib.load().pfb_spread_f64(it.handle, ctypes.c_void_p(v.data_ptr()), int(Ls),
@@ -199,7 +199,7 @@ def plan_spgram(coord, shape, basis=None, zmap=None, L=6, nbins=(40, 40), dt=Non
         # segment l weights each sample by B_l(t) of its readout position (last axis)
         bl = torch.as_tensor(bt, dtype=torch.complex128, device=dev)
         vals = vals * bl.reshape(L, *([1] * (vals.ndim - 2)), bl.shape[-1])
-        zs = zs.to(torch.complex64).contiguous()
+        zs = dense(zs.to(torch.complex64))
     scale_xyz = torch.as_tensor(osf[::-1].copy(), device=dev)
     pplan = plan_nufft(coord_t * scale_xyz, os_shape, width=width, oversamp=1.25, device=dev)
     psf = _psf_f64(vals.reshape(vals.shape[0], -1), pplan, os_shape, basis_t)
@@ -252,11 +252,11 @@ class SparseGramFunction(torch.autograd.Function):
     @staticmethod
     def forward(fctx, x, gm):
         fctx.gm = gm
-        return _gram_core(gm, x.contiguous())
+        return _gram_core(gm, dense(x))
 
     @staticmethod
     def backward(fctx, g):
-        return _gram_core(fctx.gm, g.contiguous().to(torch.complex64)), None
+        return _gram_core(fctx.gm, dense(g.to(torch.complex64))), None
 
 
 def sparse_gram(image, gram_matrix, norm=None, device="cpu", threadsperblock=128):

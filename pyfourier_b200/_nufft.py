@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._plan import NUFFTPlan, _as_tensor, plan_nufft, resolve_device, to_caller
+from ._plan import NUFFTPlan, _as_tensor, dense, plan_nufft, resolve_device, to_caller
 
 
 def norm_code(norm):
@@ -149,12 +149,12 @@ class NUFFTFunction(torch.autograd.Function):
         fctx.coord_shape = coord.shape if coord is not None else None
         if coord is not None and coord.requires_grad:
             fctx.save_for_backward(image)
-        return fwd_core(ctx, image.contiguous())
+        return fwd_core(ctx, dense(image))
 
     @staticmethod
     def backward(fctx, gy):
         ctx = fctx.ctx
-        gy = gy.contiguous().to(torch.complex64)
+        gy = dense(gy.to(torch.complex64))
         gimg = gcoord = None
         if fctx.needs_input_grad[0]:
             gimg = adj_core(ctx, gy)
@@ -162,7 +162,7 @@ class NUFFTFunction(torch.autograd.Function):
                 gimg = gimg * ctx.G  # exact adjoint of the unnormalised forward
         if fctx.needs_input_grad[1]:
             (image,) = fctx.saved_tensors
-            g = traj_grad_core(ctx, image.contiguous(), gy, ctx.fac_fwd)
+            g = traj_grad_core(ctx, dense(image), gy, ctx.fac_fwd)
             gcoord = g.reshape(fctx.coord_shape)
         return gimg, gcoord, None
 
@@ -176,12 +176,12 @@ class NUFFTAdjointFunction(torch.autograd.Function):
         fctx.coord_shape = coord.shape if coord is not None else None
         if coord is not None and coord.requires_grad:
             fctx.save_for_backward(kspace)
-        return adj_core(ctx, kspace.contiguous())
+        return adj_core(ctx, dense(kspace))
 
     @staticmethod
     def backward(fctx, gx):
         ctx = fctx.ctx
-        gx = gx.contiguous().to(torch.complex64)
+        gx = dense(gx.to(torch.complex64))
         gk = gcoord = None
         if fctx.needs_input_grad[0]:
             gk = fwd_core(ctx, gx)
@@ -189,7 +189,7 @@ class NUFFTAdjointFunction(torch.autograd.Function):
                 gk = gk / ctx.G
         if fctx.needs_input_grad[1]:
             (kspace,) = fctx.saved_tensors
-            g = traj_grad_core(ctx, gx, kspace.contiguous(), ctx.fac_adj)
+            g = traj_grad_core(ctx, gx, dense(kspace), ctx.fac_adj)
             gcoord = g.reshape(fctx.coord_shape)
         return gk, gcoord, None
 
@@ -201,7 +201,7 @@ def _prep_basis(basis, dev):
     if basis is None:
         return None
     b = _as_tensor(basis)
-    return b.to(dev, torch.complex64).contiguous()
+    return dense(b.to(dev, torch.complex64))
 
 
 def _sample_shape(interp):
@@ -217,14 +217,14 @@ def _split_weight(weight, sample_shape, dev):
     w = _as_tensor(weight)
     w = w.to(dev)
     if w.dtype == torch.float32 and w.shape == sample_shape and w.is_contiguous():
-        return w.reshape(-1), None
+        return w.resolve_neg().reshape(-1), None
     if not torch.is_complex(w):
         w = w.to(torch.float32)
         lead = w.ndim - len(sample_shape)
         ws = w.reshape(w.shape[max(lead, 0):]) if lead <= 0 or all(s == 1 for s in w.shape[:lead]) else None
         if ws is not None:
             try:
-                ws = torch.broadcast_to(ws, sample_shape).reshape(-1).contiguous()
+                ws = dense(torch.broadcast_to(ws, sample_shape).reshape(-1))
                 return ws, None
             except RuntimeError:
                 pass

@@ -27,6 +27,12 @@ def _as_tensor(x, dtype=None):
     return torch.as_tensor(np.asarray(x), dtype=dtype)
 
 
+def dense(t):
+    """``t`` as a kernel reads it through its pointer: contiguous, with a lazy conjugation
+    or negation (``x.conj()`` and the gradients that pass through it) carried out."""
+    return t.resolve_conj().resolve_neg().contiguous()
+
+
 def release_cached_memory(device=None):
     """Hand the device memory kept from destroyed plans back to the driver (plans
     allocate from a pool that keeps it for the next plan); synchronises the device."""
@@ -131,7 +137,7 @@ class Interpolator:
         h = ctypes.c_void_p()
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream(self.device)
-            c = self._coord.to(self.device, torch.float32).contiguous()
+            c = dense(self._coord.to(self.device, torch.float32))
             _lib.check(L.pfb_plan_create(
                 ctypes.c_void_p(c.data_ptr()), nd, self.nframes, offs, self.readout_len,
                 _lib.int_array(self.shape), _lib.int_array(self.ishape), _lib.int_array(self.width),
@@ -320,8 +326,8 @@ def plan_nufft(coord, shape, width=4, oversamp=1.25, zmap=None, L=6, nbins=(40, 
                 raise ValueError("Please provide raster time dt if T is not known")
             T = dt * np.arange(readout, dtype=np.float32)
         b, c = mri_exp_approx(_as_tensor(zmap).to(dev), T, L, nbins)
-        zt = torch.as_tensor(b, dtype=torch.complex64, device=dev).contiguous()
-        zs = c.to(torch.complex64).contiguous()
+        zt = dense(torch.as_tensor(b, dtype=torch.complex64, device=dev))
+        zs = dense(c.to(torch.complex64))
         if L_batch_size is None:
             L_batch_size = L
     plan = NUFFTPlan(ndim, tuple(float(o) for o in oversamp), tuple(int(w) for w in width),

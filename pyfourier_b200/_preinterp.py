@@ -35,7 +35,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._plan import _as_tensor, resolve_device, to_caller
+from ._plan import _as_tensor, dense, resolve_device, to_caller
 
 
 def _operators(calib, ndim, lamda):
@@ -125,7 +125,7 @@ class GrogPlan:
             G = G[:, None]
         self.nslices = int(G.shape[1])
         self.ntable = int(G.shape[0])
-        self.table = G.to(torch.complex64).contiguous()
+        self.table = dense(G.to(torch.complex64))
         idx, lut = _lut(coord_t, nsteps)
         n_xyz = torch.tensor(shape[::-1], dtype=torch.int64, device=dev)
         ind = (idx + (n_xyz // 2).to(torch.float32)).to(torch.int64)
@@ -165,7 +165,7 @@ class GrogPlan:
         if self.nslices > 1 and B != self.nslices:
             raise ValueError(f"2D GROG with {self.nslices} calibration slices needs {self.nslices} leading input "
                              f"slices, got {B}")
-        x = x.contiguous()
+        x = dense(x)
         out = torch.empty_like(x)
         n = ctypes.c_size_t()
         _lib.check(L.pfb_grog_workspace_size(self.handle, B, ctypes.byref(n)))
