@@ -174,15 +174,15 @@ template <int MODE, int NV, bool BIG>
 int launch_nv(ColPass P, cudaStream_t s) {
     const int64_t blocks = (int64_t)P.nplanes * P.nmid * ((P.X + NV - 1) / NV);
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
-    P.T = streams(P.fa, NV);
+    const int bufs = (P.fa.nst > 2 ? 2 : 1) + (MODE == kImageOut && P.Cl ? 1 : 0);
+    const size_t smem = (size_t)bufs * ColAddr<NV>::size(P.fa.n) * sizeof(float2);
+    P.T = streams(P.fa, NV, smem, blocks);
     P.dx = Div((P.X + NV - 1) / NV);
     P.dmid = Div(P.nmid);
     P.dnch = Div(P.ch.nch);
     P.dk = Div(P.ch.K);
     P.db = Div(P.ch.B);
     P.dc = Div(P.C);
-    const int bufs = (P.fa.nst > 2 ? 2 : 1) + (MODE == kImageOut && P.Cl ? 1 : 0);
-    const size_t smem = (size_t)bufs * ColAddr<NV>::size(P.fa.n) * sizeof(float2);
     auto k = col_kernel<MODE, NV, BIG>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, NV * P.T, smem, s>>>(P);

@@ -173,14 +173,14 @@ int launch_t(GramRows P, cudaStream_t s) {
     P.nbv = std::max(1, std::min(P.batch, most / per));
     P.V = P.nbv * per;
     P.nbg = (P.batch + P.nbv - 1) / P.nbv;
-    P.T = streams(P.fa, P.V, 16);
+    const size_t smem = (size_t)2 * P.V * pitch * sizeof(float2);
+    const int64_t blocks = (int64_t)P.nbg * (!LOWRANK ? P.K : 1) * P.rows * P.nseg;
+    P.T = streams(P.fa, P.V, smem, blocks, 16);
     P.dt = Div(P.T);
     P.dbg = Div(P.nbg);
     P.dk = Div(P.K);
     P.drow = Div(P.rows);
     if (P.V * P.T > kMaxThreads) return fail(PFB_ERR_UNSUPPORTED, "Gram rows: too many threads");
-    const size_t smem = (size_t)2 * P.V * pitch * sizeof(float2);
-    const int64_t blocks = (int64_t)P.nbg * (!LOWRANK ? P.K : 1) * P.rows * P.nseg;
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
     auto k = gram_rows_kernel<LOWRANK, BIG>;
     PFB_RAISE_SMEM(k, (int)smem);

@@ -108,14 +108,26 @@ template <bool BIG>
 int launch_gram_rows_t(const GramRows &P, cudaStream_t s);
 int launch_row(const RowPass &P, bool inv, cudaStream_t s);
 
-// Threads per vector of a CTA with nv vectors: the count (64 to kMaxThreads threads) that
-// leaves the fewest thread slots idle over the stages' rounds, a butterfly of radix r
-// costing about r + 2; the larger on a tie.  With a prime stage, whose items are long, the
-// count within a quarter of that which takes them in the fewest rounds (118 = 2 x 59 points,
-// y pass, 34 us with two rounds and 15 us with one); not for those above kMaxPrime, whose
-// passes are bound by throughput (167 points: 454 us by the first rule).  At least `least`
-// (row passes: lanes along the row, whole 128-byte segments).
-inline int streams(const FftAxis &fa, int nv, int least = 1) {
+// Threads per vector of a CTA with nv vectors and `smem` bytes, `blocks` of them in the
+// launch: the count (64 to kMaxThreads threads) that leaves the fewest thread slots idle
+// over the stages' rounds, a butterfly of radix r costing about r + 2, as long as the CTAs
+// that share an SM have kFullWarps warps.  With fewer (long vectors, whose CTAs shared
+// memory limits to a few per SM, or few CTAs) the latency of a warp counts instead of its
+// slots, and more threads in fewer rounds are the faster.  The larger on a tie.  By the idle
+// slots alone 624 points ran in CTAs of 64 threads, 10 warps an SM, at 15 % issue slots
+// (2D, 12 channels, a forward and an adjoint, us: 624 points 69 + 134, now 65 + 102; 640
+// points 77 + 125, now 71 + 100; 936 points 258 + 395, now 174 + 248; over 12086 calls of
+// 16 to 1024 points 1.03 times as fast, 16 warps 1.04 but 10 % slower around 400 points).
+// With a prime stage, whose items are long, the count within a quarter of that which takes
+// them in the fewest rounds (118 = 2 x 59 points, y pass, 34 us with two rounds and 15 us
+// with one); not for those above kMaxPrime, whose passes are bound by throughput (167
+// points: 454 us by the first rule).  At least `least` (row passes: lanes along the row,
+// whole 128-byte segments).
+constexpr int kFullWarps = 12;
+inline int streams(const FftAxis &fa, int nv, size_t smem, int64_t blocks, int least = 1) {
+    // CTAs per SM: shared memory (1 KB each is the system's), and the launch's share of the 148
+    const int fit = (int)std::min<int64_t>(227 * 1024 / (int64_t)(smem + 1024), (blocks + 147) / 148);
+    const int regs = min_blocks(big_plan(fa)) * kMaxThreads / 32;  // warps that the registers hold
     const int t0 = std::max(std::max(64 / nv, 1), least);
     int best = 0, rounds = 0;
     double low = 1e300, cost = 1e300;
@@ -135,7 +147,8 @@ inline int streams(const FftAxis &fa, int nv, int least = 1) {
                     c += (double)((m + t - 1) / t) * (r + 2.0);
                 }
             }
-            c *= (t * nv + 31) / 32;
+            const int warps = (t * nv + 31) / 32, ctas = std::max(1, std::min(fit, regs / warps));
+            c *= std::max((double)warps, (double)kFullWarps / ctas);
             if (pass == 0) {
                 if (c <= low) best = t, low = c;
             } else if (c <= 1.25 * low && (rounds == 0 || pr < rounds || (pr == rounds && c <= cost))) {

@@ -105,17 +105,17 @@ int launch_fwd(RowPass P, cudaStream_t s) {
     P.V = P.cpt * P.kpt;
     P.cp = P.cpt >= 8 ? P.cpt | 1 : P.cpt;  // odd pitch from 8 channels: conflict-free transposes
     P.buf = std::max(P.V * RowAddr::pitch(n), P.kpt * n * P.cp);
-    P.T = streams(P.fa, P.V, 16);
+    const size_t smem = (size_t)2 * P.buf * sizeof(float2);
+    const int64_t ngrp = P.nvec / ((int64_t)P.nch * P.nos1 * P.nos2);
+    const int64_t blocks = ngrp * P.nos2 * P.nyb * P.nchunk;
+    P.T = streams(P.fa, P.V, smem, blocks, 16);
     P.dt = Div(P.T);
     P.dchunk = Div(P.nchunk);
     P.dyb = Div(P.nyb);
     P.dz = Div(P.nos2);
     P.dcpt = Div(P.cpt);
     P.dunit = Div(P.nch % 2 == 0 && P.cpt % 2 == 0 ? P.cpt / 2 : P.cpt);
-    const int64_t ngrp = P.nvec / ((int64_t)P.nch * P.nos1 * P.nos2);
-    const int64_t blocks = ngrp * P.nos2 * P.nyb * P.nchunk;
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
-    const size_t smem = (size_t)2 * P.buf * sizeof(float2);
     auto k = row_fwd_kernel<BIG>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, P.V * P.T, smem, s>>>(P);
@@ -127,11 +127,11 @@ template <bool BIG>
 int launch_inv(RowPass P, cudaStream_t s) {
     P.V = P.fa.n > 128 ? 8 : vectors(P.fa.n, P.nvec);
     P.buf = P.V * RowAddr::pitch(P.fa.n);
-    P.T = streams(P.fa, P.V, 16);
-    P.dt = Div(P.T);
-    const int64_t blocks = (P.nvec + P.V - 1) / P.V;
-    if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
     const size_t smem = (size_t)(P.fa.nst > 2 ? 2 : 1) * P.buf * sizeof(float2);
+    const int64_t blocks = (P.nvec + P.V - 1) / P.V;
+    P.T = streams(P.fa, P.V, smem, blocks, 16);
+    P.dt = Div(P.T);
+    if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
     auto k = row_inv_kernel<BIG>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, P.V * P.T, smem, s>>>(P);
