@@ -591,23 +591,29 @@ int pfb_gram_apply(pfb_gram *g, const void *image, void *out, int64_t batch, con
     size_t wb = 0;
     int st = get_fft_plan(g->fft_mu, g->fft_plans, g->fft_work, g->ndim, g->nos, P, &h, &wb);
     if (st) return st;
+    const float2 *Cl = static_cast<const float2 *>(b0_space);
     if (gram_is_dense(g)) {
         // grid == image, one segment: FFT image -> out, mix in place with the 1/G
         // of the two transforms folded in, inverse FFT in place (3 passes, no
-        // embed / extract copies)
+        // embed / extract copies; those two only for the factors of a field map)
         if (workspace_bytes < wb) return fail(PFB_ERR_WORKSPACE, "workspace too small");
         float2 *o = static_cast<float2 *>(out);
-        if ((st = run_fft_to(g->fft_mu, h, wb, static_cast<const float2 *>(image), o, -1, workspace, workspace_bytes, s)))
-            return st;
+        if (Cl) {
+            if ((st = launch_embed(g->ndim, g->n, g->nos, static_cast<const float2 *>(image), o, bk, Cl, 1, s))) return st;
+            st = run_fft(g->fft_mu, h, wb, o, -1, workspace, workspace_bytes, s);
+        } else {
+            st = run_fft_to(g->fft_mu, h, wb, static_cast<const float2 *>(image), o, -1, workspace, workspace_bytes, s);
+        }
+        if (st) return st;
         if ((st = launch_mix(g->gvol, g->K, g->lowrank, batch, g->d_T, o, s, (float)(1.0 / (double)g->gvol))))
             return st;
-        return run_fft(g->fft_mu, h, wb, o, +1, workspace, workspace_bytes, s);
+        if ((st = run_fft(g->fft_mu, h, wb, o, +1, workspace, workspace_bytes, s)) || !Cl) return st;
+        return launch_extract(g->ndim, g->n, g->nos, o, o, bk, 1.f, Cl, 1, s);
     }
     size_t gbytes = align_up((size_t)P * g->gvol * sizeof(float2));
     if (workspace_bytes < gbytes + wb) return fail(PFB_ERR_WORKSPACE, "workspace too small");
     float2 *grid = static_cast<float2 *>(workspace);
     void *work = static_cast<char *>(workspace) + gbytes;
-    const float2 *Cl = static_cast<const float2 *>(b0_space);
     if ((st = launch_embed(g->ndim, g->n, g->nos, static_cast<const float2 *>(image), grid, bk, Cl, L, s)))
         return st;
     if ((st = run_fft(g->fft_mu, h, wb, grid, -1, work, workspace_bytes - gbytes, s))) return st;
