@@ -257,9 +257,9 @@ int pfb_nufft_traj_grad(pfb_plan *plan, const pfb_apply_t *opt, const void *imag
  *   INTERP: interleaved grid -> per-channel sample results;  OUT: results -> dst k-space
  *   VALS:   src k-space -> per-channel sample values;  SPREAD: values -> grid
  *   CROP:   grid -> dst image (cropped, deapodised, times `factor`)
- * For 2D and 3D grids whose axes are at most 1024 long, without large prime
- * factors (127; 256 on one axis of a 3D grid), the transform is the fused
- * pruned FFT: PAD, FFT and TRANSPOSE are then its three forward passes
+ * Where pfb_fft_route says so (2D and 3D grids whose axes are at most 1024
+ * long, without large prime factors), the transform is the fused pruned FFT:
+ * PAD, FFT and TRANSPOSE are then its three forward passes
  * (image -> z pass -> y pass -> x pass writing the interleaved grid; 2D: y
  * pass, nothing, x pass) and IFFT / CROP its adjoint
  * passes (x and y passes / last pass writing the image); the chain of stages
@@ -320,6 +320,12 @@ int pfb_spread_f64(pfb_plan *plan, const void *values, int nch, void *grid, void
 int pfb_gram_create(int ndim, const int *shape, const int *os_shape, int ncoeff, int lowrank,
                     int nseg, const void *kernel, int device, void *stream, pfb_gram **out);
 int pfb_gram_destroy(pfb_gram *gram);
+/* 1 in *fused when the grid os_shape of images `shape` is transformed by this
+ * library's fused passes, 0 when by cuFFT: of a NUFFT plan (gram = 0), or of a
+ * Gram operator (gram = 1) with `lowrank` mixed coefficients (0: elementwise
+ * kernel) and nseg B0 segments.  Host only; a parity aid, the results are the
+ * same up to rounding. */
+int pfb_fft_route(int ndim, const int *shape, const int *os_shape, int gram, int lowrank, int nseg, int *fused);
 int pfb_gram_workspace_size(pfb_gram *gram, int64_t batch, size_t *bytes);
 
 /* Apply: image (batch, ncoeff, *shape) -> out (same).  Zero-pad into the 2x grid,

@@ -35,7 +35,7 @@ EXPORTS = (
     "pfb_gram_workspace_size", "pfb_gram_apply", "pfb_nufft_adj_noalloc",
     "pfb_grog_create", "pfb_grog_destroy", "pfb_grog_workspace_size", "pfb_grog_apply",
     "pfb_apply_workspace_size", "pfb_nufft_traj_grad", "pfb_nufft_stage", "pfb_plan_order", "pfb_spread_f64",
-    "pfb_plan_check", "pfb_release_cached_memory",
+    "pfb_plan_check", "pfb_release_cached_memory", "pfb_fft_route",
 )
 
 
@@ -120,6 +120,7 @@ def load(path=LIB_PATH):
         "pfb_spread_f64": (i32, [vp, vp, i32, vp, vp]),
         "pfb_gram_create": (i32, [i32, P(ctypes.c_int), P(ctypes.c_int), i32, i32, i32, vp, i32, vp, P(vp)]),
         "pfb_gram_destroy": (i32, [vp]),
+        "pfb_fft_route": (i32, [i32, P(ctypes.c_int), P(ctypes.c_int), i32, i32, i32, P(ctypes.c_int)]),
         "pfb_gram_workspace_size": (i32, [vp, i64, P(ctypes.c_size_t)]),
         "pfb_gram_apply": (i32, [vp, vp, vp, i64, vp, vp, ctypes.c_size_t, vp]),
         "pfb_nufft_adj_noalloc": (i32, [vp, P(ApplyT), vp, vp, vp]),

@@ -532,10 +532,23 @@ int pfb_gram_create(int ndim, const int *shape, const int *os_shape, int ncoeff,
         delete g;
         return fail(PFB_ERR_CUDA, std::string("kernel copy: ") + cudaGetErrorString(e));
     }
-    bool dense = nseg == 1;  // the grid is the image: no pad and crop to save
-    for (int a = 0; a < ndim; ++a) dense = dense && g->n[a] == g->nos[a];
-    if (ndim >= 2) g->fused = fft_axes(ndim, g->nos, dense, g->ax, &g->d_tw);
+    const GramRoute route{g->lowrank ? ncoeff : 0, nseg};
+    g->fused = fft_axes(ndim, g->n, g->nos, &route, g->ax, &g->d_tw);
     *out = g;
+    return PFB_OK;
+}
+
+int pfb_fft_route(int ndim, const int *shape, const int *os_shape, int gram, int lowrank, int nseg, int *fused) {
+    if (!shape || !os_shape || !fused || ndim < 1 || ndim > 3 || lowrank < 0 || nseg < 1)
+        return fail(PFB_ERR_INVALID, "bad argument");
+    int n[3], nos[3];
+    for (int a = 0; a < ndim; ++a) {
+        n[a] = shape[ndim - 1 - a];
+        nos[a] = os_shape[ndim - 1 - a];
+        if (n[a] < 1 || nos[a] < n[a]) return fail(PFB_ERR_INVALID, "need 1 <= shape <= os_shape");
+    }
+    const GramRoute route{lowrank, nseg};
+    *fused = fft_route(ndim, n, nos, gram ? &route : nullptr);
     return PFB_OK;
 }
 

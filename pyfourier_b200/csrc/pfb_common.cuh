@@ -147,8 +147,7 @@ struct FftAxis {
     int twoff[kFftMaxStages] = {};
     int rootoff[kFftMaxStages] = {};
     int swapoff = 0;  // rows of two stages: the twiddles of the two radices in the other order
-    unsigned magic[kFftMaxStages] = {};    // floor(i / ns) = umulhi(i, magic) for i < 2^16 (ns > 1)
-    unsigned magic_m[kFftMaxStages] = {};  // the same for n / radix
+    unsigned magic[kFftMaxStages] = {};  // floor(i / ns) = umulhi(i, magic) for i < 2^16 (ns > 1)
     const float2 *tw = nullptr;
 };
 
@@ -432,10 +431,14 @@ void pool_free(void *p, cudaStream_t s);
 int counting_sort_pairs(const int *keys, const int *vals, int *keys_out, int *vals_out, int64_t n, int end_bit,
                         void *temp, size_t temp_bytes, cudaStream_t s);
 
-// fused pruned FFT (pfb_fft.cu).  The Gram: 1 and the axes with a device twiddle table
-// (pool memory of the current device) when every axis is taken, else 0; dense: a Gram whose
-// grid is the image.
-int fft_axes(int ndim, const int *nos, bool dense, FftAxis *ax, float2 **d_tw);
+// fused pruned FFT (pfb_fft.cu): 1 when its passes take grids nos of images n (x first), else 0
+// (library transform); gram: a Gram operator's, else a NUFFT's.  fft_axes: and the axes with a
+// device twiddle table (pool memory of the current device).
+struct GramRoute {
+    int lowrank, nseg;  // coefficients of a low-rank kernel (0: elementwise), B0 segments
+};
+int fft_route(int ndim, const int *n, const int *nos, const GramRoute *gram);
+int fft_axes(int ndim, const int *n, const int *nos, const GramRoute *gram, FftAxis *ax, float2 **d_tw);
 // Gram apply: images [plane][*n] -> out through grids of N rows (see pfb_fft_gram.cu);
 // planes = segments x batch x K; ws: gram_fused_workspace bytes
 struct GramFused {

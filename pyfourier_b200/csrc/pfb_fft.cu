@@ -87,11 +87,10 @@ bool split_smooth(int n, std::vector<int> &f) {
 // The stages of an n-point transform: two stages up to 16 where they exist, then two up to
 // 32 (in row passes, whose lanes run along the n / r butterflies of the first stage, a
 // length that also splits into three stages up to 16 only where that leaves at least 8:
-// 125 points as 25 x 5 214 us, as 5 x 5 x 5 158 us for 100^3 x 12), then more stages: the
-// radices of the part without prime factors above 13, the largest first and the next
-// largest last, around one stage per larger prime.  The first and the last stage, which
-// read and write global memory, are never such prime stages (a radix-1 stage copies).
-// False when the fused passes do not take the length.
+// 125 points as 25 x 5 214 us, as 5 x 5 x 5 158 us for 100^3 x 12), then three or more: the
+// largest radix first and the next largest last.  A prime above 13 that no pair takes is
+// the middle stage of three; the first and the last, which read and write global memory,
+// then hold the rest of the length (a radix-1 stage copies).  False when there is no such plan.
 bool stage_plan(int n, bool rows, std::vector<int> &rad) {
     if (n < 1 || n > kMaxN) return false;
     std::vector<int> primes, f;
@@ -116,20 +115,27 @@ bool stage_plan(int n, bool rows, std::vector<int> &rad) {
             return true;
         }
     }
-    rad.clear();
-    if (f.size() < 2 && !primes.empty()) {
-        // a prime stage at the start needs no twiddle pass
-        rad.push_back(1);
-        for (int p : primes) rad.push_back(p);
-        rad.push_back(f.empty() ? 1 : f[0]);
-    } else {
-        rad.push_back(f.empty() ? 1 : f[0]);
-        for (int p : primes) rad.push_back(p);
-        for (size_t i = 2; i < f.size(); ++i) rad.push_back(f[i]);
-        rad.push_back(f.size() > 1 ? f[1] : 1);
+    if (!primes.empty()) {
+        if (primes.size() > 1 || f.size() > 1) return false;
+        rad = {1, primes[0], f.empty() ? 1 : f[0]};
+        return true;
     }
+    rad = {f.empty() ? 1 : f[0]};
+    for (size_t i = 2; i < f.size(); ++i) rad.push_back(f[i]);
+    rad.push_back(f.size() > 1 ? f[1] : 1);
     return (int)rad.size() <= kFftMaxStages;
 }
+
+// the pair has a form with constants (run_two)
+constexpr bool constant_pair(int r0, int r1) {
+#define X(R0, R1) if (r0 == R0 && r1 == R1) return true;
+    PFB_FFT_TWO(X) PFB_FFT_TWO_BIG(X)
+#undef X
+    return false;
+}
+
+// The prime of a plan's prime stage, 0 without one.
+int prime_stage(const std::vector<int> &rad) { return rad.size() == 3 && rad[1] > 16 ? rad[1] : 0; }
 
 constexpr double kPi = 3.14159265358979323846;
 
@@ -156,7 +162,6 @@ bool make_axis(int n, bool rows, FftAxis *fa, std::vector<float2> &tw, size_t *b
         fa->ns[s] = ns;
         fa->twoff[s] = (int)(tw.size() - *base);
         fa->magic[s] = magic_of(ns);
-        fa->magic_m[s] = magic_of(n / r);
         for (int q = 1; q < r; ++q)
             for (int j = 0; j < ns; ++j) root((double)j * q, (double)ns * r);
         if (s > 0 && s + 1 < fa->nst && r > 16) {  // coefficients of a prime stage, see stage_prime
@@ -189,39 +194,71 @@ bool make_axis(int n, bool rows, FftAxis *fa, std::vector<float2> &tw, size_t *b
 
 }  // namespace
 
-// Where the prime stages lose to the library's transform (measured, us, library / here):
-// an axis that is itself a prime, with no part to spread over the first and last stage, when
-// two axes of a 3D grid are (16 planes of 61^3 454 / 509, 107^3 2908 / 3538, 96 x 107 x 107
-// 2100 / 2315; with one, 96 x 96 x 107, 1426 / 1290, with two of 37 245 / 233); and on the
-// dense Gram's grids, which the library transforms in place without pad and crop (128 planes
-// of 97^2 124 / 179, 127^2 224 / 252, 254^2 969 / 1043; 166^2 350 / 349, 123^2 163 / 120).
-// The 3D figures are of grids without oversampling; at 1.25, where the passes prune, the two
-// come out within 5 % (107^3, 8 coils, 1402 / 1475, 127^3 2565 / 2510).
-static bool prime_axes_lose(int ndim, const int *nos, bool dense) {
+// Which grids the passes take: those where they are the faster, of 12000 calls on grids of 16
+// to 1024 points an axis in 2D and 3D (NUFFTs of few samples, so that the transform is most of
+// the call, and Gram operators), timed on the library's transform and here.  Figures: us,
+// library / here; 2D with 12 channels, 3D with 4, 64 points on the other axes, where not said.
+//
+// - Two stages, to 1024 points: taken (640^2 forward, with the pad and transpose that the
+//   library needs, 121 / 71, adjoint 110 / 100; of all lengths the slowest are thin grids
+//   with a long z axis: 425 points, forward 174 / 134, adjoint 150 / 169).
+// - Three stages and more: their second buffer leaves few CTAs to an SM.  Taken to 768 points
+//   (735^2 194 / 117 and 189 / 146; 1000^2 239 / 198 but 227 / 291).
+// - A prime stage, O(r^2): to 512 points (561^2 101 / 102 and 100 / 135) for primes to 64 (2D
+//   1.5 times as fast, 3D 1.1 to 1.4); for primes to kMaxPrime where the stage is the axis or
+//   half of it (254^2 87 / 69 and 89 / 73; 508^2 139 / 204 and 141 / 220), in 3D the whole
+//   axis only beside axes that make up for it (83 points in y 72 / 73 and 71 / 81; 89 beside
+//   96 x 96, 6 channels, 199 / 120 and 172 / 138); for primes to kMaxPrime3 on such an axis, y
+//   or z, that is at least 1.5 times its image, so that the passes skip a third of it (111 of
+//   167 points in y, 150 x 150, 16 channels, 2129 / 1514 and 1956 / 1772; 166 of 167 points
+//   2237 / 2268 and 2148 / 2508; 115 of 173, 128 x 128, 1086 / 989 and 894 / 1113).
+//   Two axes of a 3D grid that are such primes: not (16 planes of 61^3 454 / 509, 107^3 2908 /
+//   3538; with one, 96 x 96 x 107, 1426 / 1290).
+// - A Gram whose grid is the image is transformed in place by the library, without pad and
+//   crop: taken in 2D with at most 5 coefficients, at 96 to 400 points in two stages with
+//   constants (256^2 x 4, 12 images 71 / 53, 256 images 896 / 853; elementwise 31 / 24), or with
+//   radices to 16 where the coefficients are mixed (165^2 x 4 65 / 37, elementwise 26 / 29).
+//   With 8 coefficients 256^2 takes 146 / 187 (128 images 1065 / 1693); in 3D 64^3 29 / 40,
+//   64 of them 368 / 395.
+// - A low-rank Gram holds all K planes of a row twice in shared memory: taken to 64 KB (8
+//   planes of 440 points 491 / 417, of 1024 points 1538 / 2343).
+static bool fused_takes(int ndim, const int *n, const int *nos, const GramRoute *gram) {
+    if (ndim < 2) return false;
+    bool dense = gram && gram->nseg == 1;
+    for (int a = 0; a < ndim; ++a) dense = dense && n[a] == nos[a];
+    if (dense && (ndim != 2 || gram->lowrank > 5)) return false;
     int bare = 0;
     for (int a = 0; a < ndim; ++a) {
-        int m = nos[a], p = 1;  // the largest prime factor
-        for (int d = 2; m > 1; ++d)
-            while (m % d == 0) {
-                m /= d;
-                p = d;
+        std::vector<int> rad;
+        if (!stage_plan(nos[a], a == 0, rad)) return false;
+        const int len = nos[a], p = prime_stage(rad);
+        if (dense) {
+            if (rad.size() != 2 || len < 96) return false;
+            if (!(constant_pair(rad[0], rad[1]) && len <= 400) && !(gram->lowrank > 1 && rad[0] <= 16)) return false;
+        } else if (rad.size() > 2 && !p) {
+            if (len > 768) return false;
+        } else if (p) {
+            if (len > 512) return false;
+            if (p > 48 && p == len) ++bare;
+            int64_t other = 1;
+            for (int b = 0; b < ndim; ++b) other *= b == a ? 1 : nos[b];
+            if (p > 64) {
+                if (p > kMaxPrime ? ndim == 2 || p != len || a == 0 || 2 * (int64_t)len < 3 * (int64_t)n[a] : len > 2 * p)
+                    return false;
+                if (ndim == 3 && p == len && other < 96 * 96) return false;
             }
-        if (dense && (p > 96 || (p > 32 && p == nos[a]))) return true;
-        if (p > 48 && p == nos[a]) ++bare;
+        }
     }
-    return ndim == 3 && bare >= 2;
+    if (ndim == 3 && bare >= 2) return false;
+    // two buffers of K rows
+    return !gram || 2 * gram->lowrank * RowAddr::pitch(nos[0]) * (int)sizeof(float2) <= 64 * 1024;
 }
 
-int fft_axes(int ndim, const int *nos, bool dense, FftAxis *ax, float2 **d_tw) {
+int fft_route(int ndim, const int *n, const int *nos, const GramRoute *gram) { return fused_takes(ndim, n, nos, gram) ? 1 : 0; }
+
+int fft_axes(int ndim, const int *n, const int *nos, const GramRoute *gram, FftAxis *ax, float2 **d_tw) {
     *d_tw = nullptr;
-    int large = 0;  // axes with a prime factor above kMaxPrime
-    for (int a = 0; a < ndim; ++a) {
-        std::vector<int> rad;
-        if (!stage_plan(nos[a], a == 0, rad)) return 0;
-        for (int r : rad)
-            if (r > kMaxPrime) ++large;
-    }
-    if (large > (ndim == 3 ? 1 : 0) || prime_axes_lose(ndim, nos, dense)) return 0;
+    if (!fused_takes(ndim, n, nos, gram)) return 0;
     std::vector<float2> tw;
     size_t base[3] = {0, 0, 0};
     for (int a = 0; a < ndim; ++a)
@@ -241,7 +278,7 @@ int fft_fused_ready(pfb_plan *p) {
     std::lock_guard<std::mutex> lk(p->fft_mu);
     if (p->fft_fused >= 0) return p->fft_fused;
     p->fft_fused = 0;
-    if (p->g.ndim < 2 || !fft_axes(p->g.ndim, p->g.nos, false, p->fft_ax, &p->d_fft_tw)) return 0;
+    if (!fft_axes(p->g.ndim, p->g.n, p->g.nos, nullptr, p->fft_ax, &p->d_fft_tw)) return 0;
     // the TMA passes' flag and persistent grid (optional: without them the direct passes run)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||

@@ -26,12 +26,9 @@
 namespace pfb {
 namespace fft {
 
-// Largest prime factor: the O(r^2) stage loses to the library's transform above it (96
-// channels of 64 x 127: both directions 70 us here, 71 us there; 64 x 139: 88 against 53).
-// One axis of a 3D grid may have one up to kMaxPrime3: the other axes' passes and the pad,
-// crop and transpose kernels they replace outweigh it (93 x 111 x 120 at osf 1.5, 167 points
-// in y, 5 coils: 1098 against 1444 us).
-constexpr int kMaxPrime = 127, kMaxPrime3 = 256;
+// Largest primes of a prime stage: above kMaxPrime the O(r^2) stage loses to the library's
+// transform, but for an outer axis of a 3D grid up to kMaxPrime3 (measured beside fused_takes).
+constexpr int kMaxPrime = 127, kMaxPrime3 = 167;
 
 // cos and sin of 2 pi m / n for m = 0..n-1, evaluated at compile time (Taylor series in
 // double after reduction to the first eighth of the circle)
@@ -328,9 +325,9 @@ __device__ __forceinline__ void stage_last(int n, const float2 *__restrict__ tw,
     }
 }
 
-// A stage whose radix is a prime that no two-stage plan takes: the twiddles are applied in
-// place, then a thread takes kPrimeOut pairs of outputs (k, r - k) of a butterfly and walks
-// the (r - 1) / 2 input pairs.  The table `rt` holds its coefficients in that order as
+// A stage whose radix is a prime that no two-stage plan takes, after a radix-1 stage (so
+// without twiddles): a thread takes kPrimeOut pairs of outputs (k, r - k) of a butterfly and
+// walks the (r - 1) / 2 input pairs.  The table `rt` holds its coefficients in that order as
 // (cos, cos, sin, sin) of 2 pi q k / r, the operands of packed FMAs: per input pair and
 // output pair one 16-byte load and two FMAs, no index arithmetic (with the roots looked up
 // by q k mod r: 36 instructions for 4 output pairs instead of 16; 472 = 8 x 59 points, 31
@@ -338,22 +335,12 @@ __device__ __forceinline__ void stage_last(int n, const float2 *__restrict__ tw,
 // table of 167, 111 KB, misses L1 (y pass of 93 x 111 x 120, 5 coils: 566 us).
 constexpr int kPrimeOut = 4;
 template <bool DUP, class A>
-__device__ __forceinline__ void stage_prime(int n, int R, int ns, unsigned magic, unsigned magic_m,
-                                            const float2 *__restrict__ tw, const float2 *__restrict__ rt, int stream,
-                                            int T, A ad, float2 *__restrict__ src, float2 *__restrict__ dst) {
+__device__ __forceinline__ void stage_prime(int n, int R, const float2 *__restrict__ rt, int stream, int T, A ad,
+                                            const float2 *__restrict__ src, float2 *__restrict__ dst) {
     const int m = n / R, H = (R - 1) / 2;
-    if (ns > 1) {
-        for (int p = stream; p < n; p += T) {
-            const int q = (int)__umulhi((unsigned)p, magic_m), i = p - q * m;
-            const int j = i - (int)__umulhi((unsigned)i, magic) * ns;
-            if (q > 0) src[ad(p)] = cmul(src[ad(p)], __ldg(tw + (q - 1) * ns + j));
-        }
-        __syncthreads();
-    }
     const int ng = (H + kPrimeOut - 1) / kPrimeOut;
     for (int w = stream; w < m * ng; w += T) {
         const int g = w / m, i = w - g * m;
-        const int j = ns == 1 ? 0 : i - (int)__umulhi((unsigned)i, magic) * ns;
         const float2 x0 = src[ad(i)];
         float2 c[kPrimeOut], s[kPrimeOut], sum = x0;
 #pragma unroll
@@ -380,14 +367,14 @@ __device__ __forceinline__ void stage_prime(int n, int R, int ns, unsigned magic
                 }
             }
         }
-        const int base = (i - j) * R + j;
+        const int base = i * R;
         if (g == 0) dst[ad(base)] = sum;
 #pragma unroll
         for (int u = 0; u < kPrimeOut; ++u) {
             const int k = g * kPrimeOut + u + 1;
             if (k > H) break;
-            dst[ad(base + k * ns)] = cadd(c[u], cmi(s[u]));
-            dst[ad(base + (R - k) * ns)] = csub(c[u], cmi(s[u]));
+            dst[ad(base + k)] = cadd(c[u], cmi(s[u]));
+            dst[ad(base + R - k)] = csub(c[u], cmi(s[u]));
         }
     }
 }
@@ -493,11 +480,11 @@ __device__ __forceinline__ void run(const FftAxis &fa, int stream, int T, A ad, 
                     // share a group of outputs and its coefficients
                     const int V = blockDim.x / T, pv = threadIdx.x % V;
                     if (fa.radix[s] <= kMaxPrime)
-                        stage_prime<true>(n, fa.radix[s], ns, mg, fa.magic_m[s], tw, fa.tw + fa.rootoff[s],
-                                          threadIdx.x / V, T, A::of(pv, n), src, dst);
+                        stage_prime<true>(n, fa.radix[s], fa.tw + fa.rootoff[s], threadIdx.x / V, T, A::of(pv, n), src,
+                                          dst);
                     else
-                        stage_prime<false>(n, fa.radix[s], ns, mg, fa.magic_m[s], tw, fa.tw + fa.rootoff[s],
-                                           threadIdx.x / V, T, A::of(pv, n), src, dst);
+                        stage_prime<false>(n, fa.radix[s], fa.tw + fa.rootoff[s], threadIdx.x / V, T, A::of(pv, n), src,
+                                           dst);
                     break;
                 }
             }
