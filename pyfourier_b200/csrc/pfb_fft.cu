@@ -216,9 +216,10 @@ bool make_axis(int n, bool rows, FftAxis *fa, std::vector<float2> &tw, size_t *b
 //   3538; with one, 96 x 96 x 107, 1426 / 1290).
 // - A Gram whose grid is the image is transformed in place by the library, without pad and
 //   crop: taken in 2D with at most 5 coefficients, at 96 to 400 points in two stages with
-//   constants (256^2 x 4, 12 images 71 / 53, 256 images 896 / 853; elementwise 31 / 24), or with
-//   radices to 16 where the coefficients are mixed (165^2 x 4 65 / 37, elementwise 26 / 29).
-//   With 8 coefficients 256^2 takes 146 / 187 (128 images 1065 / 1693); in 3D 64^3 29 / 40,
+//   constants (256^2 x 4, 12 images 71 / 53, 256 images 896 / 853; elementwise 31 / 24) and to
+//   288 points without, where the last radix is not small (1.05 to 1.3 times as fast by the
+//   number of images and coefficients; single images of 3 MB from 0.85 to 1.3; 27 x 9 points
+//   0.8, 17 x 17 0.9).  With 8 coefficients 256^2 takes 146 / 187 (128 images 1065 / 1693); in 3D 64^3 29 / 40,
 //   64 of them 368 / 395.
 // - A low-rank Gram holds all K planes of a row twice in shared memory: taken to 64 KB (8
 //   planes of 440 points 491 / 417, of 1024 points 1538 / 2343).
@@ -234,7 +235,8 @@ static bool fused_takes(int ndim, const int *n, const int *nos, const GramRoute 
         const int len = nos[a], p = prime_stage(rad);
         if (dense) {
             if (rad.size() != 2 || len < 96) return false;
-            if (!(constant_pair(rad[0], rad[1]) && len <= 400) && !(gram->lowrank > 1 && rad[0] <= 16)) return false;
+            if (!(constant_pair(rad[0], rad[1]) && len <= 400) && !(len <= 288 && (rad[0] <= 16 || rad[1] >= 10)))
+                return false;
         } else if (rad.size() > 2 && !p) {
             if (len > 768) return false;
         } else if (p) {

@@ -46,7 +46,7 @@ def test_large_primes_on_an_outer_axis(os, shape, want):
 @pytest.mark.parametrize("os, lowrank, want", [
     ((256, 256), 0, 1), ((256, 256), 4, 1), ((256, 256), 5, 1), ((256, 256), 6, 0), ((256, 256), 8, 0),
     ((64, 64), 0, 0), ((96, 96), 3, 1), ((384, 384), 4, 1), ((500, 500), 4, 0), ((512, 512), 0, 0),
-    ((125, 125), 4, 0), ((243, 243), 4, 0), ((165, 165), 0, 0), ((165, 165), 4, 1), ((97, 97), 0, 0),
+    ((125, 125), 4, 0), ((243, 243), 4, 0), ((165, 165), 0, 1), ((272, 272), 4, 1), ((289, 289), 4, 0), ((97, 97), 0, 0),
     ((64, 64, 64), 0, 0), ((128, 128, 128), 4, 0),
 ])
 def test_gram_grids_of_the_images_size(os, lowrank, want):
