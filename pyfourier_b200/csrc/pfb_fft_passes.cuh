@@ -109,7 +109,8 @@ int launch_gram_rows_t(const GramRows &P, cudaStream_t s);
 int launch_row(const RowPass &P, bool inv, cudaStream_t s);
 
 // Threads per vector of a CTA with nv vectors and `smem` bytes, `blocks` of them in the
-// launch: the count (64 to kMaxThreads threads) that leaves the fewest thread slots idle
+// launch: the count (64 to kMaxThreads threads; from 32 for a vector alone, the Gram rows of a
+// single image: 96^3 on 192^3 133 -> 95 us) that leaves the fewest thread slots idle
 // over the stages' rounds, a butterfly of radix r costing about r + 2, as long as the CTAs
 // that share an SM have kFullWarps warps.  With fewer (long vectors, whose CTAs shared
 // memory limits to a few per SM, or few CTAs) the latency of a warp counts instead of its
@@ -128,7 +129,7 @@ inline int streams(const FftAxis &fa, int nv, size_t smem, int64_t blocks, int l
     // CTAs per SM: shared memory (1 KB each is the system's), and the launch's share of the 148
     const int fit = (int)std::min<int64_t>(227 * 1024 / (int64_t)(smem + 1024), (blocks + 147) / 148);
     const int regs = min_blocks(big_plan(fa)) * kMaxThreads / 32;  // warps that the registers hold
-    const int t0 = std::max(std::max(64 / nv, 1), least);
+    const int t0 = std::max((nv == 1 ? 32 : 64) / nv, std::max(least, 1));
     int best = 0, rounds = 0;
     double low = 1e300, cost = 1e300;
     bool has_prime = false;
