@@ -407,16 +407,18 @@ __device__ __forceinline__ void run_two(const float2 *__restrict__ tw, int strea
     }
 }
 
-// The lengths with constants: those of image extents in steps of 8 and 16 at the usual
-// oversampling factors and of their doubled (Toeplitz) grids, in the plans that
-// stage_plan picks.  Runtime indices cost the row passes as many instructions as the
-// transform itself (256 points: 50 a point and transform against about 28).
+// The lengths with constants, in the plans that stage_plan picks: image extents of 64 to 256
+// in steps of 16 or 20 at the oversampling factors 1, 1.25 and 1.5 and doubled (Toeplitz
+// grids), from 80 points on, where row passes take two stages.  Runtime indices cost the row
+// passes as many instructions as the transform itself (256 points: 50 a point and transform
+// against about 28).
 #define PFB_FFT_TWO(X) \
-    X(12, 8) X(10, 10) X(14, 8) X(12, 10) X(16, 8) X(12, 12) X(15, 10) X(16, 10) X(16, 11) X(15, 12) X(16, 12) \
-    X(16, 13) X(16, 14) X(16, 15) X(16, 16)
+    X(10, 8) X(12, 8) X(10, 10) X(14, 8) X(12, 10) X(16, 8) X(14, 10) X(12, 12) X(15, 10) X(16, 10) X(14, 12) X(16, 11) \
+    X(15, 12) X(16, 12) X(16, 13) X(15, 14) X(16, 14) X(15, 15) X(16, 15) X(16, 16)
 #define PFB_FFT_TWO_BIG(X) \
-    X(20, 10) X(18, 12) X(22, 10) X(25, 10) X(25, 11) X(18, 16) X(20, 15) X(20, 16) X(22, 16) X(20, 18) X(24, 16) \
-    X(20, 20) X(22, 20) X(24, 20) X(32, 16)
+    X(20, 10) X(18, 12) X(20, 11) X(25, 10) X(20, 13) X(22, 12) X(18, 15) X(25, 11) X(20, 14) X(18, 16) X(20, 15) \
+    X(24, 13) X(20, 16) X(22, 15) X(21, 16) X(22, 16) X(20, 18) X(24, 16) X(20, 20) X(26, 16) X(22, 20) X(28, 16) \
+    X(24, 20) X(32, 16)
 
 // Forward transform of the thread's vector: points through ld(position), results through
 // st(frequency, value).  b0 and b1 (b1 only with more than two stages): A::size(n) float2
