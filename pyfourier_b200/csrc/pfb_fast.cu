@@ -1755,8 +1755,7 @@ int upload(const std::vector<T> &h, T **d) {
     }
     const int st = pool_alloc(reinterpret_cast<void **>(d), std::max<size_t>(h.size(), 1) * sizeof(T));
     if (st) return st;
-    if (!h.empty()) PFB_CUDA_TRY(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return PFB_OK;
+    return h.empty() ? PFB_OK : upload_table(*d, h.data(), h.size() * sizeof(T));
 }
 
 }  // namespace

@@ -267,7 +267,7 @@ int fft_axes(int ndim, const int *n, const int *nos, const GramRoute *gram, FftA
         if (!make_axis(nos[a], a == 0, &ax[a], tw, &base[a])) return 0;
     if (tw.empty()) tw.push_back(make_float2(1.f, 0.f));
     if (pool_alloc(reinterpret_cast<void **>(d_tw), tw.size() * sizeof(float2)) != PFB_OK) return 0;
-    if (cudaMemcpy(*d_tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload_table(*d_tw, tw.data(), tw.size() * sizeof(float2)) != PFB_OK) {
         pool_free(*d_tw, 0);
         *d_tw = nullptr;
         return 0;
@@ -288,7 +288,7 @@ int fft_fused_ready(pfb_plan *p) {
         p->fft_nsm = 0;
     if (pool_alloc(reinterpret_cast<void **>(&p->d_fft_err), sizeof(int)) != PFB_OK) {
         p->d_fft_err = nullptr;
-    } else if (cudaMemset(p->d_fft_err, 0, sizeof(int)) != cudaSuccess) {
+    } else if (clear_table(p->d_fft_err, sizeof(int)) != PFB_OK) {
         pool_free(p->d_fft_err, 0);
         p->d_fft_err = nullptr;
     }

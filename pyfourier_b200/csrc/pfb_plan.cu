@@ -249,10 +249,8 @@ int rebuild_items(pfb_plan *p, int chunk) {
     int st;
     if ((st = dev_alloc(&p->d_items_frame, a.size()))) return st;
     if ((st = dev_alloc(&p->d_items_all, b.size()))) return st;
-    if (!a.empty())
-        PFB_CUDA_TRY(cudaMemcpy(p->d_items_frame, a.data(), a.size() * sizeof(SpreadItem), cudaMemcpyHostToDevice));
-    if (!b.empty())
-        PFB_CUDA_TRY(cudaMemcpy(p->d_items_all, b.data(), b.size() * sizeof(SpreadItem), cudaMemcpyHostToDevice));
+    if (!a.empty() && (st = upload_table(p->d_items_frame, a.data(), a.size() * sizeof(SpreadItem)))) return st;
+    if (!b.empty() && (st = upload_table(p->d_items_all, b.data(), b.size() * sizeof(SpreadItem)))) return st;
     p->n_items_frame = (int)a.size();
     p->n_items_all = (int)b.size();
     p->chunk = chunk;
@@ -441,7 +439,7 @@ int plan_create(const float *coord, int ndim, int nframes, const int64_t *frame_
             vf[i] = std::isnan(r) ? 1.0f : (float)r;
         }
         PFB_TRY_ST(dev_alloc(&p->d_apod[a], n));
-        PFB_TRY_CU(cudaMemcpy(p->d_apod[a], vf.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+        PFB_TRY_ST(upload_table(p->d_apod[a], vf.data(), n * sizeof(float)));
     }
 
     int maxbin = 0;

@@ -61,6 +61,21 @@ void pool_free(void *p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
 }
 
+// A copy from pageable memory may return with its last transfer still in flight on the legacy
+// stream, and a memset always may: streams created non-blocking (torch's side streams) are not
+// ordered behind it.
+int upload_table(void *dst, const void *src, size_t bytes) {
+    PFB_CUDA_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    PFB_CUDA_TRY(cudaStreamSynchronize(0));
+    return PFB_OK;
+}
+
+int clear_table(void *dst, size_t bytes) {
+    PFB_CUDA_TRY(cudaMemset(dst, 0, bytes));
+    PFB_CUDA_TRY(cudaStreamSynchronize(0));
+    return PFB_OK;
+}
+
 }  // namespace pfb
 
 extern "C" int pfb_release_cached_memory(int device) {
