@@ -335,12 +335,13 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD && D == 3 ? 2 : 3) gather_ro
 // 6.64 ms against 5.13 ms).
 template <int D, int WM, bool WIDE, int CH, bool GRAD>
 __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(const Gather P) {
-    constexpr int NR = D == 3 ? WM * WM : WM, REC = tap_rec(D, WM), DW = D * WM;
-    constexpr int RB = WM == 4 ? 4 : 2;  // rows in flight
+    constexpr int NR = D == 3 ? WM * WM : (D == 2 ? WM : 1), REC = tap_rec(D, WM), DW = D * WM;
+    constexpr int RB = D == 1 ? 1 : (WM == 4 ? 4 : 2);  // rows in flight
+    constexpr int NG = GRAD && D > 1 ? NR : 1;
+    constexpr bool GY = GRAD && D > 1, GZ = GRAD && D > 2;  // gradients besides x
     constexpr int NW = (NR + 31) / 32;
     constexpr int NB = GRAD ? 32 / DW : 1;  // consecutive samples of a warp (gradient weights of all at once)
-    constexpr int NG = GRAD ? NR : 1;
-    static_assert(REC <= 32 && NR % RB == 0 && D >= 2, "one record word per lane, whole batches of rows");
+    static_assert(REC <= 32 && NR % RB == 0, "one record word per lane, whole batches of rows");
     __shared__ __align__(16) float s_rec[kWarps][32];
     __shared__ __align__(16) int s_px[kWarps][8];
     __shared__ __align__(16) int s_roff[kWarps][NR];
@@ -388,15 +389,15 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(
             const int t = lane + 32 * k;
             if (t < NR) {
                 const int iy = t % WM, iz = t / WM;
-                const bool ok = iy < P.g.w[1] && (D < 3 || iz < P.g.w[2]);
-                float w = 0.f, wy = 0.f, wz = 0.f;
+                const bool ok = D == 1 || (iy < P.g.w[1] && (D < 3 || iz < P.g.w[2]));
+                float w = D == 1 ? 1.f : 0.f, wy = 0.f, wz = 0.f;
                 int off = 0;
-                if (ok) {
+                if (D > 1 && ok) {
                     const float vz = D > 2 ? rw[2 * WM + iz] : 1.f;
                     w = rw[WM + iy] * vz;
-                    if (GRAD) wy = rd[WM + iy] * vz;
-                    if (GRAD && D > 2) wz = rw[WM + iy] * rd[2 * WM + iz];
-                    off = tap_pos(first_pos(x0[1], P.g.sh[1], P.g.nos[1]), iy, P.g.nos[1]) * P.g.nos[0];
+                    if (GY) wy = rd[WM + iy] * vz;
+                    if (GZ) wz = rw[WM + iy] * rd[2 * WM + iz];
+                    off = tap_pos(first_pos(x0[D > 1 ? 1 : 0], P.g.sh[1], P.g.nos[1]), iy, P.g.nos[1]) * P.g.nos[0];
                     if (D > 2)
                         off += tap_pos(first_pos(x0[D > 2 ? 2 : 0], P.g.sh[2], P.g.nos[2]), iz, P.g.nos[2]) *
                                (P.g.nos[0] * P.g.nos[1]);
@@ -404,8 +405,8 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(
                 }
                 s_roff[warp][t] = off;
                 s_rw[warp][t] = make_float2(w, w);
-                if constexpr (GRAD) s_ry[warp][t] = make_float2(wy, wy);
-                if constexpr (GRAD && D > 2) s_rz[warp][t] = make_float2(wz, wz);
+                if constexpr (GY) s_ry[warp][t] = make_float2(wy, wy);
+                if constexpr (GZ) s_rz[warp][t] = make_float2(wz, wz);
             }
         }
         __syncwarp();
@@ -422,12 +423,12 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(
 #pragma unroll
                 for (int u = 0; u < WM; ++u) px[u] = s_px[warp][u];
             }
-            float2 ax[WM], bx[GRAD ? WM : 1], cx[GRAD && D > 2 ? WM : 1];
+            float2 ax[WM], bx[GY ? WM : 1], cx[GZ ? WM : 1];
 #pragma unroll
             for (int u = 0; u < WM; ++u) {
                 ax[u] = make_float2(0.f, 0.f);
-                if constexpr (GRAD) bx[u] = ax[u];
-                if constexpr (GRAD && D > 2) cx[u] = ax[u];
+                if constexpr (GY) bx[u] = ax[u];
+                if constexpr (GZ) cx[u] = ax[u];
             }
             auto run = [&](auto addr) {
 #pragma unroll
@@ -437,9 +438,11 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(
                     if constexpr (RB == 4) {
                         const int4 o4 = reinterpret_cast<const int4 *>(s_roff[warp])[rb];
                         o[0] = o4.x, o[1] = o4.y, o[2] = o4.z, o[3] = o4.w;
-                    } else {
+                    } else if constexpr (RB == 2) {
                         const int2 o2 = reinterpret_cast<const int2 *>(s_roff[warp])[rb];
                         o[0] = o2.x, o[1] = o2.y;
+                    } else {
+                        o[0] = 0;  // 1D: the one row
                     }
 #pragma unroll
                     for (int q = 0; q < RB; ++q) {
@@ -451,12 +454,12 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(
                         const float2 wr = s_rw[warp][rb * RB + q];
 #pragma unroll
                         for (int u = 0; u < WM; ++u) ax[u] = __ffma2_rn(wr, v[q * WM + u], ax[u]);
-                        if constexpr (GRAD) {
+                        if constexpr (GY) {
                             const float2 wy = s_ry[warp][rb * RB + q];
 #pragma unroll
                             for (int u = 0; u < WM; ++u) bx[u] = __ffma2_rn(wy, v[q * WM + u], bx[u]);
                         }
-                        if constexpr (GRAD && D > 2) {
+                        if constexpr (GZ) {
                             const float2 wz = s_rz[warp][rb * RB + q];
 #pragma unroll
                             for (int u = 0; u < WM; ++u) cx[u] = __ffma2_rn(wz, v[q * WM + u], cx[u]);
@@ -479,10 +482,10 @@ __global__ void __launch_bounds__(kWarps * 32, GRAD ? 2 : 3) gather_xrow_kernel(
             for (int u = 0; u < WM; ++u) {
                 const float w = u < P.g.w[0] ? (GRAD ? rd : rw)[u] : 0.f;
                 d0 = __ffma2_rn(make_float2(w, w), ax[u], d0);
-                if constexpr (GRAD) {
+                if constexpr (GY) {
                     const float wx = u < P.g.w[0] ? rw[u] : 0.f;
                     d1 = __ffma2_rn(make_float2(wx, wx), bx[u], d1);
-                    if constexpr (D > 2) d2 = __ffma2_rn(make_float2(wx, wx), cx[u], d2);
+                    if constexpr (GZ) d2 = __ffma2_rn(make_float2(wx, wx), cx[u], d2);
                 }
             }
             if (c < nch) {
@@ -535,12 +538,17 @@ int launch_t(Gather &P, cudaStream_t s) {
     // chunks of at most 32 / w0 units, as even as they go
     const int most = 32 / w0;
     P.nchunk = (P.nu + most - 1) / most;
-    if constexpr (D >= 2 && WM >= 4) {
-        // a channel per lane above 16 channels, and where the rows take more than one
-        // chunk (2D) or two (3D): 2D width 6, 16 channels 132 us against 106, 3D width 6,
-        // 15 channels 1114 against 857, but 3D width 4, 15 channels 775 against 890 and
-        // width 6, 16 channels 733 against 857
-        if (P.ch.nch > 16 || P.nchunk > (D == 3 ? 2 : 1)) return launch_xrow<D, WM, GRAD>(P, s);
+    if constexpr (WM >= 4) {
+        // a channel per lane above 16 channels, and where the rows take too many chunks, us as
+        // rows / channel per lane.  1D, one row: more than one chunk (512 k samples, width 4, 24
+        // channels 195 / 140; width 6, 16 channels 201 / 140, 31 channels 428 / 168).  2D: two
+        // of widths 7 and 8 and of an odd count at widths 5 and 6 (512 k samples, width 8, 5
+        // channels 264 / 407, 16 channels 401 / 426, 15 channels in four 612 / 425; width 6, 9
+        // channels 258 / 276, 16 channels 320 / 287; width 4, 15 channels 207 / 196), and any
+        // of the gradient (102 k samples, width 8, 16 channels 131 / 162).  3D: two (width 6, 15
+        // channels 1114 / 857, 16 channels 733 / 857, width 4, 15 channels 775 / 890)
+        const int most_chunks = D == 1 ? 1 : D == 3 ? 2 : GRAD ? 8 : WM == 8 || (WM == 6 && !pair) ? 2 : 1;
+        if (P.ch.nch > 16 || P.nchunk > most_chunks) return launch_xrow<D, WM, GRAD>(P, s);
     }
     P.cpv = (P.nu + P.nchunk - 1) / P.nchunk;
     P.U = w0 * P.cpv;
