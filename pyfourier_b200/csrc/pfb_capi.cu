@@ -247,7 +247,7 @@ int pfb_plan_set_chunk(pfb_plan *p, int chunk) {
     DeviceGuard dg(p->device);
     int st = rebuild_items(p, chunk);
     if (st) return st;
-    return build_owner_items(p, chunk);
+    return build_owner_items(p, chunk, false);
 }
 
 int pfb_plan_tables(const pfb_plan *p, int axis, int32_t *index, float *value, void *stream) {

@@ -408,7 +408,8 @@ int fast_traj_grad(pfb_plan *p, const ApplyDesc &d, const float2 *img, const flo
                    size_t wsb, float factor, bool accumulate, cudaStream_t s);
 int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void *dst, void *ws, size_t wsb,
                float factor, bool accumulate, cudaStream_t s);
-int build_owner_items(pfb_plan *p, int chunk);
+// even: tiles that are all about equally full stay whole up to twice the chunk
+int build_owner_items(pfb_plan *p, int chunk, bool even);
 // gather.cu: interleaved grid -> results of the sorted samples [M][nch]; the trajectory
 // gradient (values vt [M][B], weight applied)
 int launch_interp_il(const pfb_plan *p, const Chan &c, const float2 *grid, float2 *res, cudaStream_t s);

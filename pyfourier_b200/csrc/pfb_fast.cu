@@ -1746,6 +1746,28 @@ void owner_items_for(const pfb_plan *p, bool per_frame, int chunk, std::vector<O
     }
 }
 
+// Splitting shortens the chain of a crowded tile.  Where no tile is crowded (the fullest has at
+// most twice the mean) it only adds set-ups, zeroing and atomics: tiles of at most twice the
+// chunk then stay whole (3D, uniform samples, 60^3, us, split / whole: 51 k samples x 32
+// channels width 4 202 / 180, width 6 304 / 258, 8 channels 142 / 134, 26 k x 32 217 / 190).
+// Fuller ones gain from the split with few channels (205 k x 1 224 / 237, 1.02 M x 8 813 / 1026).
+void keep_even_tiles(int chunk, std::vector<OwnerItem> &items, std::vector<OwnerItem> &zero) {
+    long long sum = 0, n = 0;
+    int most = 0;
+    for (const OwnerItem &i : items)
+        if ((!i.atomic || i.v0 == 0) && i.v1 > 0) {
+            sum += i.v1;
+            ++n;
+            most = std::max(most, i.v1);
+        }
+    if (zero.empty() || most > std::min(2LL * chunk, 4096LL) || most * n > 2 * sum) return;
+    size_t k = 0;
+    for (const OwnerItem &i : items)
+        if (!i.atomic || i.v0 == 0) items[k++] = {i.tile, i.frame, 0, i.v1, 0};
+    items.resize(k);
+    zero.clear();
+}
+
 template <typename T>
 int upload(const std::vector<T> &h, T **d) {
     if (*d) {
@@ -1760,15 +1782,17 @@ int upload(const std::vector<T> &h, T **d) {
 
 }  // namespace
 
-int build_owner_items(pfb_plan *p, int chunk) {
+int build_owner_items(pfb_plan *p, int chunk, bool even) {
     std::vector<OwnerItem> it, z;
     int st;
     owner_items_for(p, true, chunk, it, z);
+    if (even) keep_even_tiles(chunk, it, z);
     if ((st = upload(it, &p->d_own_frame))) return st;
     if ((st = upload(z, &p->d_zero_frame))) return st;
     p->n_own_frame = (int)it.size();
     p->n_zero_frame = (int)z.size();
     owner_items_for(p, false, chunk, it, z);
+    if (even) keep_even_tiles(chunk, it, z);
     if ((st = upload(it, &p->d_own_all))) return st;
     if ((st = upload(z, &p->d_zero_all))) return st;
     p->n_own_all = (int)it.size();
