@@ -5,8 +5,8 @@ the samples and the owner tile of the spread) and the number of samples per
 spread work item, by timing a forward + adjoint NUFFT on synthetic data with
 CUDA events.  The best choice is cached on disk per problem signature (GPU
 name, dimensions, oversampled grid, kernel widths, sample count bucket,
-frames, batch, coefficients, B0 segments), so later plans of the same problem
-reuse it without timing.
+frames, batch, coefficients, B0 segments, kernel generation), so later plans
+of the same problem reuse it without timing.
 
 Cache file: ``$PYFOURIER_B200_CACHE`` or ``~/.cache/pyfourier_b200/autotune.json``.
 """
@@ -48,13 +48,18 @@ def _save_cache(cache):
         pass  # a read-only home directory only disables the cache
 
 
+# Counted up when a kernel or a default changes, so that choices timed on earlier kernels are
+# timed again (2: visits per item by the number of samples, 2D register tiles from 9 channels)
+_KERNELS = 2
+
+
 def signature(plan, batch, ncoeff, nseg):
     ip = plan.interpolator
     mb = int(round(math.log2(max(ip.total_samples, 1))))
     return "|".join([
         torch.cuda.get_device_name(plan.device), f"d{ip.ndim}", "os" + "x".join(map(str, ip.ishape)),
         "w" + "x".join(map(str, ip.width)), f"m2^{mb}", f"f{ip.nframes}", f"b{batch}", f"c{ncoeff}",
-        f"l{nseg}"])
+        f"l{nseg}", f"k{_KERNELS}"])
 
 
 def default_candidates(ndim):

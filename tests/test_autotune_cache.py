@@ -41,3 +41,20 @@ def test_default_candidates():
         tiles, chunks = _autotune.default_candidates(ndim)
         assert tiles and all(len(t) == ndim and all(e >= 1 for e in t) for t in tiles)
         assert chunks and all(1 <= c <= 16384 for c in chunks)  # pfb_plan_set_chunk's range
+
+
+def test_choices_of_earlier_kernels_are_not_used(tmp_path, monkeypatch):
+    """A cache entry without the kernel generation (as written before there was one) is a miss."""
+    import types
+
+    import torch
+
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda d: "B200")
+    ip = types.SimpleNamespace(total_samples=8000000, ndim=3, ishape=(250,) * 3, width=(4,) * 3, nframes=1)
+    plan = types.SimpleNamespace(interpolator=ip, device="cuda:0")
+    key = _autotune.signature(plan, 32, 1, 1)
+    monkeypatch.setenv("PYFOURIER_B200_CACHE", str(tmp_path / "autotune.json"))
+    _autotune._save_cache({"B200|d3|os250x250x250|w4x4x4|m2^23|f1|b32|c1|l1": {"tile": [8, 8, 8], "chunk": 2048}})
+    assert key not in _autotune._load_cache()
+    monkeypatch.setattr(_autotune, "_KERNELS", _autotune._KERNELS + 1)
+    assert _autotune.signature(plan, 32, 1, 1) != key
