@@ -1057,7 +1057,7 @@ __device__ __forceinline__ void reg2_rows(float2 (&acc)[32], const float2 (&wx2)
 // spread_reg3_kernel.  Eight blocks of 4 (x) x 8 (y) points tile the packed
 // 16 x 16 tile; a lane group of CPW channels owns one block, its 32 points x
 // its lane's channel in registers (no atomics), so a CTA has 8 / (32 / CPW)
-// warps and 2 (32 channels), 3 (16) or 4 (8) CTAs share an SM.  A sample's tile
+// warps and 2 (32 channels) or 3 (16) CTAs share an SM.  A sample's tile
 // weights are 16 x-weights and 16 y-weights (lanes (axis, t) build them), its
 // occupancy mask holds x in bits 0..15 and y in bits 16..31.
 constexpr int kReg2Tile = 16;
@@ -1066,8 +1066,8 @@ template <int CPW, int REC>
 struct Reg2Cfg {
     static constexpr int G = 32 / CPW;
     static constexpr int NW = 8 / G;
-    static constexpr int MinBlocks = CPW == 32 ? 2 : (CPW == 16 ? 3 : 4);
-    static constexpr int Batch = CPW == 32 ? 96 : (CPW == 16 ? 96 : 80);
+    static constexpr int MinBlocks = CPW == 32 ? 2 : 3;
+    static constexpr int Batch = 96;
     static constexpr size_t OffR = (size_t)Batch * CPW * sizeof(float2);
     static constexpr size_t OffD = OffR + (size_t)Batch * REC * sizeof(int);
     static constexpr size_t Buf = OffD + (size_t)Batch * sizeof(int);

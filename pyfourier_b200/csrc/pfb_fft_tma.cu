@@ -474,21 +474,15 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
     }
     int k = 0;
-    bool store_pending = false;  // thread 0: a TMA store of the scratch buffer may still be reading it
     for (int t = blockIdx.x; t < P.ntiles; t += gridDim.x, ++k) {
         const int s = k & 1;
         bool ok = mbar_wait(&full[s], (k >> 1) & 1);
         float2 *S = tsm + s * P.slot;
-        if (threadIdx.x == 0 && store_pending) {
-            bulk_wait_read0();
-            store_pending = false;
-        }
         ok = __syncthreads_and(ok);
         if (!ok) {
             if (threadIdx.x == 0) {
                 atomicExch(P.err, 1);
                 if (t + (int)gridDim.x < P.ntiles) mbar_wait(&full[s ^ 1], ((k + 1) >> 1) & 1);
-                if (store_pending) bulk_wait_read0();
             }
             return;
         }
@@ -507,14 +501,12 @@ __global__ void __launch_bounds__(kThreads, 2)
             const int kz = r % P.nos2, grp = r / P.nos2;
             tma_store4(&dst_map, chn0, 0, kz * P.nos1 + ky, grp, R);
             bulk_commit();
-            // refill the slot now unless the store reads it; a store of the scratch
-            // buffer is waited for before the next transform
-            if (R == S) bulk_wait_read0();
-            else store_pending = true;
+            // a two-stage transform leaves its result in the slot: refill it once the store
+            // has read it
+            bulk_wait_read0();
             if (tn < P.ntiles) issue(tn, s);
         }
     }
-    if (threadIdx.x == 0 && store_pending) bulk_wait_read0();
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (the driver

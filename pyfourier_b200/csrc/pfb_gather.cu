@@ -560,8 +560,8 @@ int launch_t(Gather &P, cudaStream_t s) {
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(need, 148LL * 64));
     const bool wide = P.g.gvol * (int64_t)P.nu >= (1LL << 31);
     // few rows in 2D: two chunks keep enough loads in flight (the gradient has no registers
-    // left for the second one)
-    constexpr int NC1 = GRAD ? 1 : 2, NC2 = D == 3 ? 1 : NC1;
+    // left for the second one; 1D has one chunk)
+    constexpr int NC1 = GRAD || (D == 1 && WM >= 4) ? 1 : 2, NC2 = D == 3 ? 1 : NC1;
     auto run = [&](auto k) { k<<<blocks, kWarps * 32, 0, s>>>(P); };
     if (pair && wide) run(gather_rows_kernel<D, WM, 2, true, GRAD, 1>);
     else if (wide) run(gather_rows_kernel<D, WM, 1, true, GRAD, 1>);
