@@ -247,7 +247,8 @@ int pfb_plan_set_chunk(pfb_plan *p, int chunk) {
     DeviceGuard dg(p->device);
     int st = rebuild_items(p, chunk);
     if (st) return st;
-    return build_owner_items(p, chunk, false);
+    if ((st = build_owner_items(p, chunk, false))) return st;
+    return wait_tables();
 }
 
 int pfb_plan_tables(const pfb_plan *p, int axis, int32_t *index, float *value, void *stream) {
@@ -535,7 +536,7 @@ int pfb_gram_create(int ndim, const int *shape, const int *os_shape, int ncoeff,
     const GramRoute route{g->lowrank ? ncoeff : 0, nseg};
     g->fused = fft_axes(ndim, g->n, g->nos, &route, g->ax, &g->d_tw);
     *out = g;
-    return PFB_OK;
+    return wait_tables();
 }
 
 int pfb_fft_route(int ndim, const int *shape, const int *os_shape, int gram, int lowrank, int nseg, int *fused) {

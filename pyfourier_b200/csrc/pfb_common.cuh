@@ -429,10 +429,11 @@ size_t counting_sort_temp_bytes(int64_t n);
 // use, or synchronises the device first).
 int pool_alloc(void **p, size_t bytes);
 void pool_free(void *p, cudaStream_t s);
-// Host table -> device memory, and zeroed device memory, that every stream may read on return
-// (plan time)
+// Host table -> device memory, and zeroed device memory (plan time); every stream may read them
+// once wait_tables has returned, which an entry point that makes tables calls before it does
 int upload_table(void *dst, const void *src, size_t bytes);
 int clear_table(void *dst, size_t bytes);
+int wait_tables();
 int counting_sort_pairs(const int *keys, const int *vals, int *keys_out, int *vals_out, int64_t n, int end_bit,
                         void *temp, size_t temp_bytes, cudaStream_t s);
 

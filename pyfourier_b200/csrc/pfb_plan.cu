@@ -452,6 +452,7 @@ int plan_create(const float *coord, int ndim, int nframes, const int64_t *frame_
     // twiddle tables of the fused transform now, so that no apply allocates
     // (applies may be captured into CUDA graphs)
     fft_fused_ready(p);
+    PFB_TRY_ST(wait_tables());
 #undef PFB_TRY_ST
 #undef PFB_TRY_CU
     cleanup(PFB_OK);
