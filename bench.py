@@ -635,9 +635,24 @@ def time_device(torch, fn, steps, warmup):
     return a.elapsed_time(b) / steps
 
 
-def stage_bytes(plan, B, C=1, L=1, basis=False):
+def touched_points(torch, interp):
+    """Grid points that some tap of the frame reads, summed over the frames (2D plans)."""
+    (iy, _), (ix, _) = interp.tables(0), interp.tables(1)
+    iy, ix = iy.reshape(-1, iy.shape[-1]).long(), ix.reshape(-1, ix.shape[-1]).long()
+    ny, nx = interp.ishape
+    total = 0
+    for a, b in zip(interp.frame_offsets[:-1], interp.frame_offsets[1:]):
+        hit = torch.zeros(ny * nx, dtype=torch.bool, device=iy.device)
+        hit[(iy[a:b, :, None] * nx + ix[a:b, None, :]).reshape(-1)] = True
+        total += int(hit.sum())
+    return total
+
+
+def stage_bytes(plan, B, C=1, L=1, basis=False, touched=None):
     """Bytes each stage of the channel-interleaved pipeline must move at minimum
-    (inputs read once, outputs written once), 2D or 3D.
+    (inputs read once, outputs written once), 2D or 3D.  ``touched``: the grid points that
+    the interpolation reads over all frames, where the samples leave some out (few views a
+    frame: counting the whole grid put its rate above the memory's).
 
     B batch, C coefficients (K with a basis, else frames), L B0 segments.  Image
     planes: B C; grid planes: B C L; channels per sample: B L (x K with a basis).
@@ -654,7 +669,8 @@ def stage_bytes(plan, B, C=1, L=1, basis=False):
     nch = B * L * (C if basis else 1)
     img = B * C * int(np.prod(Ns)) * 8
     gp = B * C * L * 8
-    out = {"interp": gp * G + nch * M * 8 + coords, "out": nch * M * 8 + B * M * 8,
+    read = gp * G if touched is None else B * L * 8 * touched
+    out = {"interp": read + nch * M * 8 + coords, "out": nch * M * 8 + B * M * 8,
            "vals": B * M * 8 + nch * M * 8, "spread": nch * M * 8 + gp * G + coords}
     if nd == 3:
         a = Ns[0] * Ns[1] * ns[2]       # after the z pass
@@ -841,7 +857,8 @@ def wl_cfg4(torch, pf, dev, args, clocks, cpu=True):
     del graph
     stages = stage_times(torch, pf, bplan, x, 5)
     peak, peak_kind = measured_hbm_peak()
-    roof = stage_roofline(stages, stage_bytes(bplan, B, F, Lseg), peak, peak_kind)
+    roof = stage_roofline(stages, stage_bytes(bplan, B, F, Lseg, touched=touched_points(torch, bplan.interpolator)), peak,
+                          peak_kind)
     out = {"metric": "B0-corrected NUFFT fwd+adj samples/s, batched graph-captured (2D radial, 64 uneven frames)",
            "value": B * Mtot / (ms_graph / 1e3), "unit": "samples/s", "ms_per_step": ms_graph,
            "steps": args.steps, "warmup": args.warmup,

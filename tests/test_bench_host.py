@@ -172,3 +172,20 @@ def test_exact_off_resonance_model():
     ref = np.array([np.sum(x * np.exp(-2j * np.pi * (c[m, 0] * xx / N + c[m, 1] * yy / N + t[m] * b0)))
                     for m in range(30)])
     assert np.abs(got - ref).max() / np.abs(ref).max() < 1e-12
+
+
+def test_stage_bytes_counts_the_grid_points_that_are_read():
+    """With the points that some tap reads, the interpolation is not charged for the others."""
+    import types
+
+    import torch
+
+    # two frames of two samples on a 6 x 8 grid, 2 taps an axis (tables in sample order)
+    iy = torch.tensor([[0, 1], [0, 1], [5, 0], [2, 3]])
+    ix = torch.tensor([[0, 1], [1, 2], [7, 0], [7, 0]])
+    interp = types.SimpleNamespace(ishape=(6, 8), frame_offsets=(0, 2, 4), tables=lambda a: ((iy, ix)[a], None))
+    assert bench.touched_points(torch, interp) == 6 + 8
+    plan = _fake_plan((4, 6), (6, 8), 4)
+    whole, part = bench.stage_bytes(plan, 3, 2, 5), bench.stage_bytes(plan, 3, 2, 5, touched=14)
+    assert whole["interp"] - part["interp"] == 3 * 5 * 8 * (2 * 48 - 14)
+    assert {k: v for k, v in whole.items() if k != "interp"} == {k: v for k, v in part.items() if k != "interp"}
