@@ -30,7 +30,9 @@ def _as_tensor(x, dtype=None):
 def dense(t):
     """``t`` as a kernel reads it through its pointer: contiguous, with a lazy conjugation
     or negation (``x.conj()`` and the gradients that pass through it) carried out."""
-    return t.resolve_conj().resolve_neg().contiguous()
+    if t.is_conj() or t.is_neg():
+        t = t.resolve_conj().resolve_neg()
+    return t.contiguous()
 
 
 def release_cached_memory(device=None):

@@ -448,11 +448,12 @@ int plan_create(const float *coord, int ndim, int nframes, const int64_t *frame_
     int chunk = ndim == 3 ? 256 : 512;
     PFB_TRY_ST(rebuild_items(p, chunk));
     PFB_TRY_ST(build_owner_items(p, default_visits(ndim, mtot), true));
-    PFB_TRY_ST(build_plan_taps(p, stream));
     // twiddle tables of the fused transform now, so that no apply allocates
     // (applies may be captured into CUDA graphs)
     fft_fused_ready(p);
     PFB_TRY_ST(wait_tables());
+    // last: the caller's host work goes on beside its kernel
+    PFB_TRY_ST(build_plan_taps(p, stream));
 #undef PFB_TRY_ST
 #undef PFB_TRY_CU
     cleanup(PFB_OK);
