@@ -29,7 +29,12 @@ namespace fft {
 
 template <int MODE>
 static int launch_col_direct(const ColPass &P, cudaStream_t s) {
-    return big_plan(P.fa) ? launch_col_mode<MODE, true>(P, s) : launch_col_mode<MODE, false>(P, s);
+    switch (plan_group(P.fa)) {
+        case 0: return launch_col_mode<MODE, 0>(P, s);
+        case 1: return launch_col_mode<MODE, 1>(P, s);
+        case 2: return launch_col_mode<MODE, 2>(P, s);
+        default: return launch_col_mode<MODE, 3>(P, s);
+    }
 }
 
 int launch_col(const ColPass &P, int mode, cudaStream_t s) {
@@ -46,7 +51,12 @@ int launch_col(const ColPass &P, int mode, cudaStream_t s) {
 
 int launch_gram_rows(const GramRows &P, cudaStream_t s) {
     if (P.batch == 0 || P.rows == 0) return PFB_OK;
-    return big_plan(P.fa) ? launch_gram_rows_t<true>(P, s) : launch_gram_rows_t<false>(P, s);
+    switch (plan_group(P.fa)) {
+        case 0: return launch_gram_rows_t<0>(P, s);
+        case 1: return launch_gram_rows_t<1>(P, s);
+        case 2: return launch_gram_rows_t<2>(P, s);
+        default: return launch_gram_rows_t<3>(P, s);
+    }
 }
 
 }  // namespace fft

@@ -256,9 +256,15 @@ struct RowAddr {
     static __host__ __device__ __forceinline__ constexpr int between(int r) { return r | 1; }
 };
 
-// the radices of a kernel's stages: 1 to 16, and those above it that only kernels with
-// BIG take (as the first of exactly two stages: 64 registers hold the points of the
-// others, 128 theirs)
+// A kernel takes the plans of one group, by the first radix: those to 12 with all plans of
+// three and more stages, 13 to 16, and above 16 (as the first of exactly two stages) to 22 and
+// to 32.  One switch over all pairs gave every pair the registers of the worst: at 64 a thread
+// the image passes reloaded 1000 to 1200 bytes of spills (700 in the first group now, 4 in the
+// second), and a pair that joined slowed others (180 points x 256, last pass, 25.6 us, 27.8
+// with five more pairs, 24.2 now; 128 points x 16 in 2D 5.8 -> 4.7).
+constexpr int group_of(int r0) { return r0 <= 12 ? 0 : r0 <= 16 ? 1 : r0 <= 22 ? 2 : 3; }
+constexpr bool big_group(int g) { return g >= 2; }
+constexpr int group_most(int g) { return g == 0 ? 12 : g == 1 ? 16 : g == 2 ? 22 : 32; }
 #define PFB_FFT_BIG(X) \
     X(17) X(18) X(19) X(20) X(21) X(22) X(23) X(24) X(25) X(26) X(27) X(28) X(29) X(30) X(31) X(32)
 #define PFB_FFT_RADICES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
@@ -413,24 +419,24 @@ __device__ __forceinline__ void run_two(const float2 *__restrict__ tw, int strea
 // passes as many instructions as the transform itself (256 points: 50 a point and transform
 // against about 28).
 #define PFB_FFT_TWO(X) \
-    X(10, 8) X(12, 8) X(10, 10) X(14, 8) X(12, 10) X(16, 8) X(14, 10) X(12, 12) X(15, 10) X(16, 10) X(14, 12) X(16, 11) \
-    X(15, 12) X(16, 12) X(16, 13) X(15, 14) X(16, 14) X(15, 15) X(16, 15) X(16, 16)
+    X(12, 8) X(10, 10) X(14, 8) X(12, 10) X(16, 8) X(12, 12) X(15, 10) X(16, 10) X(16, 11) X(15, 12) X(16, 12) \
+    X(16, 13) X(16, 14) X(16, 15) X(16, 16) X(10, 8) X(14, 10) X(14, 12) X(15, 14) X(15, 15)
 #define PFB_FFT_TWO_BIG(X) \
-    X(20, 10) X(18, 12) X(20, 11) X(25, 10) X(20, 13) X(22, 12) X(18, 15) X(25, 11) X(20, 14) X(18, 16) X(20, 15) \
-    X(24, 13) X(20, 16) X(22, 15) X(21, 16) X(22, 16) X(20, 18) X(24, 16) X(20, 20) X(26, 16) X(22, 20) X(28, 16) \
-    X(24, 20) X(32, 16)
+    X(20, 10) X(18, 12) X(20, 11) X(25, 10) X(25, 11) X(18, 16) X(20, 15) X(20, 16) X(22, 16) X(20, 18) X(24, 16) \
+    X(20, 20) X(22, 20) X(24, 20) X(32, 16) X(20, 13) X(22, 12) X(18, 15) X(20, 14) X(24, 13) X(22, 15) X(21, 16) \
+    X(26, 16) X(28, 16)
 
 // Forward transform of the thread's vector: points through ld(position), results through
 // st(frequency, value).  b0 and b1 (b1 only with more than two stages): A::size(n) float2
 // of shared memory each, not read by any thread any more when the call begins.
-template <bool BIG, class A, class L, class S>
+template <int G, class A, class L, class S>
 __device__ __forceinline__ void run(const FftAxis &fa, int stream, int T, A ad, float2 *b0, float2 *b1, L &ld, S &st) {
     const int n = fa.n, nst = fa.nst;
-    if (BIG || nst == 2) {
+    if (G > 0 || nst == 2) {
         switch (fa.radix[0] * 32 + fa.radix[1]) {
 #define X(R0, R1) \
     case R0 * 32 + R1: \
-        if constexpr (BIG == (R0 > 16)) run_two<R0, R1>(fa.tw + fa.twoff[1], stream, T, ad, b0, ld, st); \
+        if constexpr (group_of(R0) == G) run_two<R0, R1>(fa.tw + fa.twoff[1], stream, T, ad, b0, ld, st); \
         return;
             PFB_FFT_TWO(X) PFB_FFT_TWO_BIG(X)
 #undef X
@@ -439,7 +445,7 @@ __device__ __forceinline__ void run(const FftAxis &fa, int stream, int T, A ad, 
         switch (fa.radix[0]) {
 #define X(R) \
     case R: \
-        if constexpr (BIG == (R > 16)) stage_first<R, true>(n, stream, T, ad, ld, b0); \
+        if constexpr (group_of(R) == G) stage_first<R, true>(n, stream, T, ad, ld, b0); \
         break;
             PFB_FFT_RADICES(X) PFB_FFT_BIG(X)
 #undef X
@@ -450,7 +456,7 @@ __device__ __forceinline__ void run(const FftAxis &fa, int stream, int T, A ad, 
         switch (fa.radix[1]) {
 #define X(R) \
     case R: \
-        if constexpr (BIG || R <= 16) stage_last<R, true>(n, tw, stream, T, ad, b0, st); \
+        if constexpr (R <= group_most(G)) stage_last<R, true>(n, tw, stream, T, ad, b0, st); \
         break;
             PFB_FFT_RADICES(X) PFB_FFT_BIG(X)
 #undef X
@@ -458,7 +464,7 @@ __device__ __forceinline__ void run(const FftAxis &fa, int stream, int T, A ad, 
         }
         return;
     }
-    if constexpr (!BIG) {
+    if constexpr (G == 0) {
         switch (fa.radix[0]) {
 #define X(R) \
     case R: stage_first<R, false>(n, stream, T, ad, ld, b0); break;

@@ -103,8 +103,8 @@ struct ColStoreImage {
 
 // A CTA: NV adjacent columns of one (plane, mid).  What bounds it is HBM: 200^3, 32 coils,
 // see launch_col for the rates.
-template <int MODE, int NV, bool BIG>
-__global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) col_kernel(const ColPass P) {
+template <int MODE, int NV, int G>
+__global__ void __launch_bounds__(kMaxThreads, min_blocks(big_group(G))) col_kernel(const ColPass P) {
     extern __shared__ __align__(16) float2 fsm[];
     using A = ColAddr<NV>;
     const int n = P.fa.n, T = P.T;
@@ -133,17 +133,17 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) col_kernel(const
                           xin};
         if (P.Cl) {
             ColLoadImage<true> ld{src, (int)P.in_ax * 8, n, hn, P.lin, P.apod_ax, P.Cl + (int64_t)l * P.nvol + off, a};
-            run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
+            run<G>(P.fa, stream, T, ad, b0, b1, ld, st);
         } else {
             ColLoadImage<false> ld{src, (int)P.in_ax * 8, n, hn, P.lin, P.apod_ax, nullptr, a};
-            run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
+            run<G>(P.fa, stream, T, ad, b0, b1, ld, st);
         }
     } else if constexpr (MODE == kForward || MODE == kInverse) {
         constexpr bool F = MODE == kForward;
         ColLoad<F> ld{P.src + (int64_t)plane * P.in_plane + (int64_t)mid * P.in_mid + xs, (int)P.in_ax * 8, n, hn, P.lin};
         ColStore<F> st{P.dst + (int64_t)plane * P.out_plane + (int64_t)mid * P.out_mid + x, (int)P.out_ax * 8, n, hn,
                        P.lout, xin};
-        run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
+        run<G>(P.fa, stream, T, ad, b0, b1, ld, st);
     } else {  // image plane (b, c) <- grid planes of its segments
         int c;
         const int b = P.dc.split(plane, c);
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) col_kernel(const
         if (!P.Cl) {  // one segment
             ColLoad<false> ld{src + chan(0) * P.in_plane, (int)P.in_ax * 8, n, hn, P.lin};
             ColStoreImage<false> st{dst, (int)P.out_ax * 8, n, hn, P.lout, xin, P.apod_ax, a, P.accumulate != 0};
-            run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
+            run<G>(P.fa, stream, T, ad, b0, b1, ld, st);
             return;
         }
         float2 *acc = fsm + (P.fa.nst > 2 ? 2 : 1) * A::size(n) + v;
@@ -165,12 +165,12 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) col_kernel(const
                                    P.Cl + (int64_t)l * P.nvol + off + xs, acc, NV, l == 0,
                                    l + 1 == P.ch.L};
             if (l > 0) __syncthreads();  // the previous segment's last stage has read its buffer
-            run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
+            run<G>(P.fa, stream, T, ad, b0, b1, ld, st);
         }
     }
 }
 
-template <int MODE, int NV, bool BIG>
+template <int MODE, int NV, int G>
 int launch_nv(ColPass P, cudaStream_t s) {
     const int64_t blocks = (int64_t)P.nplanes * P.nmid * ((P.X + NV - 1) / NV);
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
@@ -183,18 +183,18 @@ int launch_nv(ColPass P, cudaStream_t s) {
     P.dk = Div(P.ch.K);
     P.db = Div(P.ch.B);
     P.dc = Div(P.C);
-    auto k = col_kernel<MODE, NV, BIG>;
+    auto k = col_kernel<MODE, NV, G>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, NV * P.T, smem, s>>>(P);
     PFB_CHECK_LAUNCH();
     return PFB_OK;
 }
 
-template <int MODE, bool BIG>
+template <int MODE, int G>
 int launch_col_mode(const ColPass &P, cudaStream_t s) {
     const int64_t tiles = (int64_t)P.nplanes * P.nmid * ((P.X + 15) / 16);
-    if constexpr (BIG) return launch_nv<MODE, 8, true>(P, s);
-    else return narrow_tiles(P.fa.n, tiles) ? launch_nv<MODE, 8, false>(P, s) : launch_nv<MODE, 16, false>(P, s);
+    if constexpr (big_group(G)) return launch_nv<MODE, 8, G>(P, s);
+    else return narrow_tiles(P.fa.n, tiles) ? launch_nv<MODE, 8, G>(P, s) : launch_nv<MODE, 16, G>(P, s);
 }
 
 }  // namespace fft

@@ -4,10 +4,14 @@
 namespace pfb {
 namespace fft {
 
-template int launch_col_mode<kImageIn, true>(const ColPass &, cudaStream_t);
-template int launch_col_mode<kForward, true>(const ColPass &, cudaStream_t);
-template int launch_col_mode<kInverse, true>(const ColPass &, cudaStream_t);
-template int launch_col_mode<kImageOut, true>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kImageIn, 2>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kImageIn, 3>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kForward, 2>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kForward, 3>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kInverse, 2>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kInverse, 3>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kImageOut, 2>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kImageOut, 3>(const ColPass &, cudaStream_t);
 
 }  // namespace fft
 }  // namespace pfb

@@ -4,7 +4,8 @@
 namespace pfb {
 namespace fft {
 
-template int launch_col_mode<kImageIn, false>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kImageIn, 0>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kImageIn, 1>(const ColPass &, cudaStream_t);
 
 }  // namespace fft
 }  // namespace pfb

@@ -4,7 +4,8 @@
 namespace pfb {
 namespace fft {
 
-template int launch_col_mode<kInverse, false>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kInverse, 0>(const ColPass &, cudaStream_t);
+template int launch_col_mode<kInverse, 1>(const ColPass &, cudaStream_t);
 
 }  // namespace fft
 }  // namespace pfb

@@ -4,7 +4,8 @@
 namespace pfb {
 namespace fft {
 
-template int launch_gram_rows_t<false>(const GramRows &, cudaStream_t);
+template int launch_gram_rows_t<0>(const GramRows &, cudaStream_t);
+template int launch_gram_rows_t<1>(const GramRows &, cudaStream_t);
 
 }  // namespace fft
 }  // namespace pfb

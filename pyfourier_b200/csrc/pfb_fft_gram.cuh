@@ -69,8 +69,8 @@ inline __host__ __device__ int gram_pitch(const FftAxis &fa) {
     return two > RowAddr::pitch(fa.n) ? two : RowAddr::pitch(fa.n);
 }
 
-template <bool LOWRANK, bool BIG>
-__global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) gram_rows_kernel(const GramRows P) {
+template <bool LOWRANK, int G>
+__global__ void __launch_bounds__(kMaxThreads, min_blocks(big_group(G))) gram_rows_kernel(const GramRows P) {
     extern __shared__ __align__(16) float2 fsm[];
     const int n = P.fa.n, T = P.T, N0 = P.N0, K = P.K;
     const int pitch = LOWRANK ? RowAddr::pitch(n) : gram_pitch(P.fa);
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) gram_rows_kernel
         switch (P.fa.radix[0] * 32 + P.fa.radix[1]) {
 #define X(R0, R1) \
     case R0 * 32 + R1: \
-        if constexpr (!LOWRANK && BIG == (R0 > 16)) \
+        if constexpr (!LOWRANK && group_of(R0) == G) \
             gram_two<R0, R1>(P.fa.tw + P.fa.twoff[1], P.fa.tw + P.fa.swapoff, tr, stream, T, ad, B0, B1, ld, st); \
         return;
             PFB_FFT_TWO(X) PFB_FFT_TWO_BIG(X)
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) gram_rows_kernel
     }
     float2 *M = P.fa.nst % 2 == 0 ? B1 : B0;  // the buffer that the last stage does not read
     auto sm = [&](int q, float2 r) { M[ad.at(q)] = r; };
-    run<BIG>(P.fa, stream, T, ad, B0, B1, ld, sm);
+    run<G>(P.fa, stream, T, ad, B0, B1, ld, sm);
     __syncthreads();
     float2 *O = M == B1 ? B0 : B1;
     if constexpr (!LOWRANK) {
@@ -160,10 +160,10 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) gram_rows_kernel
     __syncthreads();
     // inverse: the forward transform read reversed
     auto lm = [&](int p) { return O[ad.at(p)]; };
-    run<BIG>(P.fa, stream, T, ad, O == B1 ? B0 : B1, O, lm, st);
+    run<G>(P.fa, stream, T, ad, O == B1 ? B0 : B1, O, lm, st);
 }
 
-template <bool LOWRANK, bool BIG>
+template <bool LOWRANK, int G>
 int launch_t(GramRows P, cudaStream_t s) {
     const int n = P.fa.n, pitch = LOWRANK ? RowAddr::pitch(n) : gram_pitch(P.fa);
     // vectors per CTA: up to 16 while the two buffers stay within 64 KB (3 CTAs per SM),
@@ -182,16 +182,16 @@ int launch_t(GramRows P, cudaStream_t s) {
     P.drow = Div(P.rows);
     if (P.V * P.T > kMaxThreads) return fail(PFB_ERR_UNSUPPORTED, "Gram rows: too many threads");
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
-    auto k = gram_rows_kernel<LOWRANK, BIG>;
+    auto k = gram_rows_kernel<LOWRANK, G>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, P.V * P.T, smem, s>>>(P);
     PFB_CHECK_LAUNCH();
     return PFB_OK;
 }
 
-template <bool BIG>
+template <int G>
 int launch_gram_rows_t(const GramRows &P, cudaStream_t s) {
-    return P.lowrank ? launch_t<true, BIG>(P, s) : launch_t<false, BIG>(P, s);
+    return P.lowrank ? launch_t<true, G>(P, s) : launch_t<false, G>(P, s);
 }
 
 }  // namespace fft

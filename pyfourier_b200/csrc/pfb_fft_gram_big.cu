@@ -4,7 +4,8 @@
 namespace pfb {
 namespace fft {
 
-template int launch_gram_rows_t<true>(const GramRows &, cudaStream_t);
+template int launch_gram_rows_t<2>(const GramRows &, cudaStream_t);
+template int launch_gram_rows_t<3>(const GramRows &, cudaStream_t);
 
 }  // namespace fft
 }  // namespace pfb

@@ -10,7 +10,7 @@ constexpr int kMaxN = 1024;        // longest axis handled (else the library FFT
 constexpr int kMaxThreads = 256;   // threads per CTA
 // CTAs per SM that bound the registers: 64 a thread, or 128 with a radix above 16
 constexpr int min_blocks(bool big) { return big ? 2 : 4; }
-inline bool big_plan(const FftAxis &fa) { return fa.nst == 2 && fa.radix[0] > 16; }
+inline int plan_group(const FftAxis &fa) { return fa.nst == 2 ? group_of(fa.radix[0]) : 0; }
 
 // Division of 0 <= e < 2^31 by a divisor known at the launch, as a multiply-high and a
 // shift.  A CTA of the direct passes lives for one tile, 16 points or so a thread: a handful
@@ -102,9 +102,9 @@ int launch_col_tma(const ColPass &P, int pass, cudaStream_t s);
 int launch_row_tma(const RowPass &P, bool inv, cudaStream_t s);
 int launch_col(const ColPass &P, int mode, cudaStream_t s);
 // one instantiation per file (pfb_fft_cols_*.cu, pfb_fft_gram*.cu), so that they compile side by side
-template <int MODE, bool BIG>
+template <int MODE, int G>
 int launch_col_mode(const ColPass &P, cudaStream_t s);
-template <bool BIG>
+template <int G>
 int launch_gram_rows_t(const GramRows &P, cudaStream_t s);
 int launch_row(const RowPass &P, bool inv, cudaStream_t s);
 
@@ -114,7 +114,7 @@ int launch_row(const RowPass &P, bool inv, cudaStream_t s);
 // over the stages' rounds, a butterfly of radix r costing about r + 2, as long as the CTAs
 // that share an SM have kFullWarps warps.  With fewer (long vectors, whose CTAs shared
 // memory limits to a few per SM, or few CTAs) the latency of a warp counts instead of its
-// slots, and more threads in fewer rounds are the faster.  The larger on a tie.  By the idle
+// slots, and more threads in fewer rounds are the faster.  By the idle
 // slots alone 624 points ran in CTAs of 64 threads, 10 warps an SM, at 15 % issue slots
 // (2D, 12 channels, a forward and an adjoint, us: 624 points 69 + 134, now 65 + 102; 640
 // points 77 + 125, now 71 + 100; 936 points 258 + 395, now 174 + 248; over 12086 calls of
@@ -128,32 +128,35 @@ constexpr int kFullWarps = 12;
 inline int streams(const FftAxis &fa, int nv, size_t smem, int64_t blocks, int least = 1) {
     // CTAs per SM: shared memory (1 KB each is the system's), and the launch's share of the 148
     const int fit = (int)std::min<int64_t>(227 * 1024 / (int64_t)(smem + 1024), (blocks + 147) / 148);
-    const int regs = min_blocks(big_plan(fa)) * kMaxThreads / 32;  // warps that the registers hold
+    const int regs = min_blocks(big_group(plan_group(fa))) * kMaxThreads / 32;  // warps that the registers hold
     const int t0 = std::max((nv == 1 ? 32 : 64) / nv, std::max(least, 1));
-    int best = 0, rounds = 0;
-    double low = 1e300, cost = 1e300;
+    int best = 0, rounds = 0, width = 0;
+    double low = 1e300, cost = 1e300, steps = 0;
     bool has_prime = false;
     for (int pass = 0; pass < 2; ++pass) {
         for (int t = t0; t * nv <= kMaxThreads || best == 0; ++t) {
-            double c = 0;
+            double n = 0;  // steps of a thread, one after the other
             int pr = 0;
             for (int s = 0; s < fa.nst; ++s) {
                 const int r = fa.radix[s], m = fa.n / r;
                 if (r > 16 && s > 0 && s + 1 < fa.nst) {  // pairs of outputs in groups of 4, r / 2 steps each
                     const int w = m * (((r - 1) / 2 + 3) / 4);
-                    c += (double)((w + t - 1) / t) * (2.0 * r);
+                    n += (double)((w + t - 1) / t) * (2.0 * r);
                     pr += (w + t - 1) / t;
                     has_prime = has_prime || r <= kMaxPrime;
                 } else {
-                    c += (double)((m + t - 1) / t) * (r + 2.0);
+                    n += (double)((m + t - 1) / t) * (r + 2.0);
                 }
             }
             const int warps = (t * nv + 31) / 32, ctas = std::max(1, std::min(fit, regs / warps));
-            c *= std::max((double)warps, (double)kFullWarps / ctas);
-            if (pass == 0) {
-                if (c <= low) best = t, low = c;
-            } else if (c <= 1.25 * low && (rounds == 0 || pr < rounds || (pr == rounds && c <= cost))) {
-                best = t, rounds = pr, cost = c;
+            const double c = n * std::max((double)warps, (double)kFullWarps / ctas);
+            // on a tie the fewer steps, and more threads only within the same warps
+            const bool tie = n < steps || (n == steps && warps == width);
+            if (pass == 0 ? c < low || (c == low && tie)
+                          : c <= 1.25 * low && (rounds == 0 || pr < rounds || (pr == rounds && (c < cost || (c == cost && tie))))) {
+                if (pass == 0) low = c;
+                else rounds = pr;
+                best = t, cost = c, steps = n, width = warps;
             }
         }
         if (!has_prime) break;

@@ -10,8 +10,8 @@ namespace {
 // [grp][kz][ky][kx][ch].  A CTA holds cpt channels of kpt rows ky of one (grp, kz), so
 // that what it writes is whole runs of channels (all of a row's memory when it holds all channels);
 // the transform leaves through shared memory, channels side by side.
-template <bool BIG>
-__global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) row_fwd_kernel(const RowPass P) {
+template <int G>
+__global__ void __launch_bounds__(kMaxThreads, min_blocks(big_group(G))) row_fwd_kernel(const RowPass P) {
     extern __shared__ __align__(16) float2 fsm[];
     using A = RowAddr;
     const int n = P.fa.n, T = P.T, N0 = P.N0;
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) row_fwd_kernel(c
     auto st = [&](int k, float2 r) {
         if (on) out[(yl * n + k) * cp + c] = r;
     };
-    run<BIG>(P.fa, stream, T, ad, b0, b1, ld, st);
+    run<G>(P.fa, stream, T, ad, b0, b1, ld, st);
     __syncthreads();
     // copy-out: a thread keeps its unit (a channel, or a pair where that is 16-byte aligned)
     // and walks kx
@@ -63,8 +63,8 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) row_fwd_kernel(c
 }
 
 // inverse: rows of the planar grid (n long) -> rows of T cropped to N0
-template <bool BIG>
-__global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) row_inv_kernel(const RowPass P) {
+template <int G>
+__global__ void __launch_bounds__(kMaxThreads, min_blocks(big_group(G))) row_inv_kernel(const RowPass P) {
     extern __shared__ __align__(16) float2 fsm[];
     using A = RowAddr;
     const int n = P.fa.n, T = P.T;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kMaxThreads, min_blocks(BIG)) row_inv_kernel(c
         const int o = (int)min((unsigned)c, (unsigned)(c - n));  // mod n
         if (on && o < P.N0) dst[o] = r;
     };
-    run<BIG>(P.fa, stream, T, ad, fsm, fsm + P.buf, ld, st);
+    run<G>(P.fa, stream, T, ad, fsm, fsm + P.buf, ld, st);
 }
 
 // Vectors per CTA: 16, or 8 where two buffers of 16 take more than 48 KB (fewer than 4
@@ -91,7 +91,7 @@ int vectors(int n, int64_t nvec) {
     return 2 * 16 * RowAddr::pitch(n) * (int)sizeof(float2) > 48 * 1024 || nvec < 16 * 296 ? 8 : 16;
 }
 
-template <bool BIG>
+template <int G>
 int launch_fwd(RowPass P, cudaStream_t s) {
     const int n = P.fa.n, most = vectors(n, P.nvec);
     // channels per tile: all of them up to `most`, else the most even split (in pairs when
@@ -116,14 +116,14 @@ int launch_fwd(RowPass P, cudaStream_t s) {
     P.dcpt = Div(P.cpt);
     P.dunit = Div(P.nch % 2 == 0 && P.cpt % 2 == 0 ? P.cpt / 2 : P.cpt);
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
-    auto k = row_fwd_kernel<BIG>;
+    auto k = row_fwd_kernel<G>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, P.V * P.T, smem, s>>>(P);
     PFB_CHECK_LAUNCH();
     return PFB_OK;
 }
 
-template <bool BIG>
+template <int G>
 int launch_inv(RowPass P, cudaStream_t s) {
     P.V = P.fa.n > 128 ? 8 : vectors(P.fa.n, P.nvec);
     P.buf = P.V * RowAddr::pitch(P.fa.n);
@@ -132,7 +132,7 @@ int launch_inv(RowPass P, cudaStream_t s) {
     P.T = streams(P.fa, P.V, smem, blocks, 16);
     P.dt = Div(P.T);
     if (blocks >= (1LL << 31)) return fail(PFB_ERR_UNSUPPORTED, "too many vectors for the fused FFT");
-    auto k = row_inv_kernel<BIG>;
+    auto k = row_inv_kernel<G>;
     PFB_RAISE_SMEM(k, (int)smem);
     k<<<(unsigned)blocks, P.V * P.T, smem, s>>>(P);
     PFB_CHECK_LAUNCH();
@@ -145,8 +145,12 @@ int launch_row(const RowPass &P, bool inv, cudaStream_t s) {
     if (P.nvec == 0) return PFB_OK;
     const int st = launch_row_tma(P, inv, s);
     if (st) return st == 1 ? PFB_OK : st;
-    if (big_plan(P.fa)) return inv ? launch_inv<true>(P, s) : launch_fwd<true>(P, s);
-    return inv ? launch_inv<false>(P, s) : launch_fwd<false>(P, s);
+    switch (plan_group(P.fa)) {
+        case 0: return inv ? launch_inv<0>(P, s) : launch_fwd<0>(P, s);
+        case 1: return inv ? launch_inv<1>(P, s) : launch_fwd<1>(P, s);
+        case 2: return inv ? launch_inv<2>(P, s) : launch_fwd<2>(P, s);
+        default: return inv ? launch_inv<3>(P, s) : launch_fwd<3>(P, s);
+    }
 }
 
 }  // namespace fft
