@@ -189,3 +189,24 @@ def test_stage_bytes_counts_the_grid_points_that_are_read():
     whole, part = bench.stage_bytes(plan, 3, 2, 5), bench.stage_bytes(plan, 3, 2, 5, touched=14)
     assert whole["interp"] - part["interp"] == 3 * 5 * 8 * (2 * 48 - 14)
     assert {k: v for k, v in whole.items() if k != "interp"} == {k: v for k, v in part.items() if k != "interp"}
+
+
+def test_first_launch_trace_that_misses_kernels(monkeypatch):
+    import contextlib
+
+    import torch
+
+    launched, lost = [], [2, 0]
+    cuda = torch.autograd.DeviceType.CUDA
+    kernel = lambda n: types.SimpleNamespace(name=n, device_type=cuda)  # noqa: E731
+
+    @contextlib.contextmanager
+    def profile(activities):
+        launched.clear()
+        n = lost.pop(0)
+        yield types.SimpleNamespace(events=lambda: launched[n:])
+
+    monkeypatch.setattr(torch.profiler, "profile", profile)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    step = ["pfb::fft::col_kernel", "pfb::fft::gram_rows_kernel", "Memcpy DtoD", "torch_kernel"]
+    assert bench.count_launches(torch, lambda: launched.extend(map(kernel, step))) == (2, 3)
