@@ -1612,8 +1612,8 @@ int fast_stage(pfb_plan *p, const ApplyDesc &d, int stage, const void *src, void
                 // 8 channels 123 us against 160 us, 12 channels 167 against 134 us, 16
                 // channels 175 against 136 us and, with width 6, 311 against 162 us; adjoints of
                 // 9 to 16 channels, shared atomics against registers: 205 k to 1 M uniform,
-                // radial and spiral samples 1.5 to 2.5 times as long, 20 k 1.0 to 1.6, but 20 k
-                // spiral samples at width 4 0.87 to 0.95)
+                // radial and spiral samples 1.5 to 2.5 times as long; 20 k, where the host path
+                // bounds both at width 4, 55 us against 50 to 62 and, with width 6, 1.2 to 1.6)
                 switch (wmv) {
                     case 1: return launch_spread_reg2_w<1>(S, nitems, c.nch, s);
                     case 4: return launch_spread_reg2_w<4>(S, nitems, c.nch, s);
